@@ -33,6 +33,8 @@ constexpr int kSd = 14;            // per-slot double arrays (bp::rz .. bp::tol)
 constexpr uint32_t kLongRow = 128;
 constexpr uint32_t kChunkNnz = 512;
 
+constexpr int kTailMaxK = 4;       // widest batch whose narrow last levels go to a cluster launch
+
 enum fin_mode : int { kFinSpmv = 0, kFinXr = 1, kFinZsum = 2, kFinRz = 3, kFinResid = 4, kFinVerify = 5 };
 
 // Device pointers and settings of a batch.
@@ -948,6 +950,7 @@ struct apxb_batch {
     const double* inv_scale2 = nullptr;
     apxb::sweep_ctl* ctl = nullptr;
     int grid32 = 0;
+    apxb::tail_plan tail[2];   // cluster tails of the plans
     // operator (combined, permuted) and permutation
     const int32_t *a_ptr = nullptr, *a_idx = nullptr;
     const double* a_val = nullptr;
@@ -1026,6 +1029,7 @@ struct apxb_batch {
         a.idx = idx[dir]; a.val = val[dir]; a.ctl = ctl + dir;
         a.chunk = chunk[dir]; a.n_chunks = n_chunks[dir];
         a.val16 = val16[dir]; a.diag16 = diag16; a.in_scale2 = dir == 1 ? inv_scale2 : nullptr;
+        a.tail = tail[dir].rows ? &tail[dir] : nullptr;
         if (dir == 0) { a.in = rhs32; a.out = Yf; a.reset = Zf; }
         else { a.in = Yf; a.out = Zf; a.reset = Yf; }
     }
@@ -1334,6 +1338,16 @@ int apxb_batch_create(apxb_engine* e, int n_inst, apxb_factor* const* factors, a
         // instance sweeps over its fp32 values)
         bt->fp16 = true;
         for (const apxb_factor* f : fs) bt->fp16 = bt->fp16 && f->precision == APXB_PREC_FP16 && f->h.fp16;
+        // The narrow last levels go to a cluster launch in batches of one instance and up to kTailMaxK
+        // columns. Its rows are summed by the plan's entry lanes, so an instance's bits are the same alone
+        // and beside others; from k = 8 on the plan's groups hold column lanes too and would leave most of a
+        // warp idle there, and merged plans hide the instances' chains behind one another. Forward / backward,
+        // us, tail against none: 6-regular n = 100003 k = 1 291 / 321 : 1027 / 1416, k = 4 297 / 311 :
+        // 695 / 685, k = 16 748 / 755 : 522 / 535; 64 instances of up to 40000 rows, k = 8, 977 / 833 : 464 / 494.
+        const auto set_tail = [&](int dir, const std::vector<uint32_t>& level_item, const std::vector<uint32_t>& level_chunk) {
+            if (n_inst == 1 && k <= kTailMaxK)
+                bt->tail[dir] = apxb::plan_tail(fs[0], dir, apxb::kTailRows32, level_item, level_chunk);
+        };
         if (n_inst == 1 && fs[0]->dev.on && !bt->fp16) {
             // a device-prepared factor: the plans are built on the device from its canonical arrays
             auto alloc_bytes = [&](void** q, size_t bytes) -> std::string {
@@ -1349,6 +1363,7 @@ int apxb_batch_create(apxb_engine* e, int n_inst, apxb_factor* const* factors, a
                 bt->n_items[dir] = o.n_items;
                 bt->info[dir] = o.info; bt->ord[dir] = o.ord; bt->ptr[dir] = o.ptr; bt->idx[dir] = o.idx;
                 bt->val[dir] = o.val; bt->chunk[dir] = o.chunk; bt->n_chunks[dir] = o.n_chunks;
+                set_tail(dir, o.level_item, o.level_chunk);
             }
         } else {
             for (const apxb_factor* f : fs)   // host plans read the canonical arrays on the host
@@ -1393,6 +1408,7 @@ int apxb_batch_create(apxb_engine* e, int n_inst, apxb_factor* const* factors, a
                 bt->info[dir] = info; bt->ord[dir] = ord; bt->ptr[dir] = ptr; bt->idx[dir] = idx; bt->val[dir] = val;
                 bt->val16[dir] = v16;
                 bt->chunk[dir] = chunk; bt->n_chunks[dir] = static_cast<uint32_t>(pl.chunk.size() - 1);
+                set_tail(dir, pl.level_item, pl.level_chunk);
             }
         }
         if (bt->fp16) {   // per-row diagonal and inverse scale squared of every instance, at its row offset

@@ -63,6 +63,7 @@ int apxb_engine_create(int device, apxb_engine** out) {
     APXB_CK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device));
     APXB_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
     e->vec_grid = e->num_sms * 4;
+    e->tail_cluster = apxb::tail_cluster_size();
     e->center_k = center_k_from_env();
     int rc = e->alloc(reinterpret_cast<void**>(&e->d_err), sizeof(apxb::dev_error));
     if (rc) return rc;
@@ -268,6 +269,25 @@ int apxb_prepare_host_fp16(uint32_t n, const uint32_t* colptr, const uint32_t* r
 
 // ---------------------------------------------------------------- factor
 
+}  // extern "C"
+
+apxb::tail_plan apxb::plan_tail(const apxb_factor* f, int dir, uint32_t max_rows, const std::vector<uint32_t>& level_item,
+                                const std::vector<uint32_t>& level_chunk) {
+    tail_plan t;
+    const tail_span sp = choose_tail(f->h, max_rows);
+    if (!sp.rows || !f->e->tail_cluster) return t;
+    const int32_t l = dir == 0 ? sp.level : f->h.fwd_levels - sp.level;   // the boundary in the direction's levels
+    t.cluster = f->e->tail_cluster;
+    t.chunk = level_chunk[l];
+    t.item0 = dir == 0 ? level_item[l] : 0u;
+    t.item1 = dir == 0 ? level_item.back() : level_item[l];
+    t.first = sp.first;
+    t.rows = sp.rows;
+    return t;
+}
+
+extern "C" {
+
 int apxb_factor_create(apxb_engine* e, uint32_t n, const uint32_t* colptr, const uint32_t* rowidx,
                        const float* vals, const uint32_t* perm, int sddm, const uint64_t* rounds,
                        uint32_t n_rounds, double drop_rel, int precision, apxb_factor** out) {
@@ -341,19 +361,6 @@ int apxb_factor_create(apxb_engine* e, uint32_t n, const uint32_t* colptr, const
                 APXB_CK(cudaMemcpyAsync(f->val16[dir], pl.val16.data(), 2 * pl.val16.size(), cudaMemcpyHostToDevice, s));
             else
                 APXB_CK(cudaMemcpyAsync(f->val[dir], pl.val.data(), 4 * pl.val.size(), cudaMemcpyHostToDevice, s));
-            if (pl.seg_rows) {
-                if ((rc = f->dalloc(&f->seg_row[dir], pl.seg_row.size())) ||
-                    (rc = f->dalloc(&f->seg_lvl[dir], pl.seg_lvl.size())) ||
-                    (rc = f->dalloc(&f->seg_ptr[dir], pl.seg_ptr.size())) ||
-                    (rc = f->dalloc(&f->seg_idx[dir], pl.seg_idx.size())) ||
-                    (rc = f->dalloc(&f->seg_val[dir], pl.seg_val.size())))
-                    return rc;
-                APXB_CK(cudaMemcpyAsync(f->seg_row[dir], pl.seg_row.data(), 4 * pl.seg_row.size(), cudaMemcpyHostToDevice, s));
-                APXB_CK(cudaMemcpyAsync(f->seg_lvl[dir], pl.seg_lvl.data(), 4 * pl.seg_lvl.size(), cudaMemcpyHostToDevice, s));
-                APXB_CK(cudaMemcpyAsync(f->seg_ptr[dir], pl.seg_ptr.data(), 4 * pl.seg_ptr.size(), cudaMemcpyHostToDevice, s));
-                APXB_CK(cudaMemcpyAsync(f->seg_idx[dir], pl.seg_idx.data(), 4 * pl.seg_idx.size(), cudaMemcpyHostToDevice, s));
-                APXB_CK(cudaMemcpyAsync(f->seg_val[dir], pl.seg_val.data(), 4 * pl.seg_val.size(), cudaMemcpyHostToDevice, s));
-            }
         }
         if (fp16) {
             if ((rc = f->dalloc(&f->diag16, m)) || (rc = f->dalloc(&f->inv_scale2, m))) return rc;
@@ -368,6 +375,12 @@ int apxb_factor_create(apxb_engine* e, uint32_t n, const uint32_t* colptr, const
         f->y_armed = f->z_armed = true;
         APXB_CK(cudaGetLastError());
         f->grid64 = apxb::sweep_grid64(e->num_sms);
+        f->h.tail_level_rows = apxb::tail_level_rows_setting();
+        for (int dir = 0; dir < 2; ++dir) {
+            const apxb::sweep_plan& pl = dir == 0 ? h.fwd_plan : h.bck_plan;
+            f->tail[dir][0] = apxb::plan_tail(f.get(), dir, apxb::kTailSmem / sizeof(double), pl.level_item, pl.level_chunk);
+            f->tail[dir][1] = apxb::plan_tail(f.get(), dir, apxb::kTailRows32, pl.level_item, pl.level_chunk);
+        }
         APXB_CK(cudaStreamSynchronize(s));
         e->children++;
         *out = f.release();
@@ -448,7 +461,7 @@ apxb::sweep_args<double> sweep64_args(apxb_factor* f, int dir) {
 
 // Forward: in -> Y (re-arms Z). Backward: in -> Z (re-arms Y).
 int run_sweep64(apxb_factor* f, int dir, const double* in, double* copy_out, const double* rhs_sub,
-                const int* skip) {
+                const int* skip, bool with_tail = true) {
     cudaStream_t s = f->e->stream;
     double* out = dir == 0 ? f->Y : f->Z;
     bool& armed = dir == 0 ? f->y_armed : f->z_armed;
@@ -461,6 +474,7 @@ int run_sweep64(apxb_factor* f, int dir, const double* in, double* copy_out, con
     a.copy_out = copy_out;
     a.rhs_sub = rhs_sub;
     a.skip = skip;
+    a.tail = with_tail ? tail_of(f, dir, false) : nullptr;
     apxb::launch_sweep64(dir, a, grid64_of(f), s);
     armed = false;
     other = true;
@@ -560,8 +574,10 @@ int pair_fp32(apxb_factor* f, int k, const double* d_in, double* d_out) {
     plan_args(f, 0, a);
     a.ctl = f->ctl;
     a.out = f->Yf; a.reset = f->Zf;
+    a.tail = tail_of(f, 0, true);
     apxb::launch_sweep32_from64(0, a, d_in, grid, s);
     plan_args(f, 1, a);
+    a.tail = tail_of(f, 1, true);
     a.ctl = f->ctl + 1;
     a.in = f->Yf; a.out = f->Zf; a.reset = f->Yf;
     a.in_scale2 = f->inv_scale2;   // fp16 factors: the backward reads D^-2 y'
@@ -588,6 +604,7 @@ int sweep32_one(apxb_factor* f, int dir, const double* d_in, double* d_out) {
     a.k = 1;
     a.err = f->e->d_err; a.budget_ns = f->e->budget_ns;
     plan_args(f, dir, a);
+    a.tail = tail_of(f, dir, true);
     a.ctl = f->ctl + dir;
     if (dir == 0) {
         if (!f->yf_armed) apxb::launch_fill_sent32(f->Yf, m, s);
@@ -865,9 +882,11 @@ int enqueue_apply(apxb_operator* a, apxb_factor* f, const apxb::pcg_ptrs& p, uns
     {
         apxb::sweep_args<double> fa = sweep64_args(f, 0);
         fa.in = a->r; fa.out = f->Y; fa.reset = f->Z; fa.rhs_sub = mean_in; fa.skip = skip;
+        fa.tail = tail_of(f, 0, false);
         apxb::launch_sweep64(0, fa, grid64_of(f), s);
         apxb::sweep_args<double> ba = sweep64_args(f, 1);
         ba.in = f->Y; ba.out = f->Z; ba.reset = f->Y; ba.skip = skip;
+        ba.tail = tail_of(f, 1, false);
         apxb::launch_sweep64(1, ba, grid64_of(f), s);
     }
     apxb::launch_pcg_zsum(p, s);
@@ -1041,7 +1060,7 @@ extern "C" int apxb_test_stalled_sweep(apxb_engine* e, apxb_factor* f, uint64_t 
     APXB_CK(cudaMemcpyAsync(f->ctl, &start, sizeof(start), cudaMemcpyHostToDevice, s));
     const unsigned long long saved = e->budget_ns;
     e->budget_ns = budget_ns;
-    rc = run_sweep64(f, 0, e->d_stage_a, e->d_stage_b, nullptr, nullptr);
+    rc = run_sweep64(f, 0, e->d_stage_a, e->d_stage_b, nullptr, nullptr, false);   // every level in the dataflow launch
     e->budget_ns = saved;
     APXB_CK(cudaStreamSynchronize(s));
     if (rc) { disarm(f); return rc; }

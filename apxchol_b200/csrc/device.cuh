@@ -36,6 +36,13 @@ __device__ __forceinline__ float ld_relaxed(const float* p) {
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return __uint_as_float(v);
 }
+// The same where `on` (elsewhere y stays as it is), by predicate and not by branch.
+__device__ __forceinline__ void ld_if(bool on, const double* p, double& y) {
+    unsigned long long v = static_cast<unsigned long long>(__double_as_longlong(y));
+    asm volatile("{.reg .pred q; setp.ne.u32 q, %1, 0; @q ld.relaxed.gpu.global.b64 %0, [%2];}"
+                 : "+l"(v) : "r"(static_cast<unsigned>(on)), "l"(p) : "memory");
+    y = __longlong_as_double(static_cast<long long>(v));
+}
 __device__ __forceinline__ void st_relaxed(double* p, double x) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" :: "l"(p), "l"(__double_as_longlong(x)) : "memory");
 }

@@ -26,8 +26,8 @@
 //                    up to 32 rows, entry offsets by a scan, entries re-laid
 //                    by one thread per row; the per-item tables (info, chunk)
 //                    come from per-group counts on the host
-// Factors without round sizes (topological levels), with fp16 storage or with
-// the optional serial segment keep the host path.
+// Factors without round sizes (topological levels) or with fp16 storage keep the
+// host path.
 #include <algorithm>
 #include <cstdlib>
 #include <functional>
@@ -531,7 +531,7 @@ std::string upload(dbuf& d, const T* h, size_t count, cudaStream_t s) {
 // per level, chunks of max(1, min(8, items / 4096)) items).
 struct plan_tables {
     uint32_t n_items = 0;
-    std::vector<uint32_t> base, info, chunk;
+    std::vector<uint32_t> base, info, chunk, level_item, level_chunk;
 };
 
 void make_tables(const std::vector<uint32_t>& counts /* [fwd level][cls] */, int32_t n_levels, uint32_t n_cls,
@@ -543,6 +543,8 @@ void make_tables(const std::vector<uint32_t>& counts /* [fwd level][cls] */, int
     for (int32_t ld = 0; ld < n_levels; ++ld) {
         const int32_t l = forward ? ld : n_levels - 1 - ld;
         const uint32_t level_first = items;
+        t.level_item.push_back(items);
+        t.level_chunk.push_back(static_cast<uint32_t>(t.chunk.size()));
         for (uint32_t c = 0; c < n_cls; ++c) {
             const uint32_t g = counts[static_cast<size_t>(l) * n_cls + c];
             const uint32_t lg = factor_plan ? (c == 4 ? 0u : 5u - c) : 5u - c, cap = 32u >> lg;
@@ -558,6 +560,8 @@ void make_tables(const std::vector<uint32_t>& counts /* [fwd level][cls] */, int
         const uint32_t per = std::max(1u, std::min(8u, in_level / 4096u));
         for (uint32_t s = level_first; s < items; s += per) t.chunk.push_back(s);
     }
+    t.level_item.push_back(items);
+    t.level_chunk.push_back(static_cast<uint32_t>(t.chunk.size()));
     t.chunk.push_back(items);
     t.n_items = items;
 }
@@ -609,6 +613,8 @@ std::string build_plan_dev(uint32_t m, int dir, uint32_t col_lanes, int32_t n_le
     out = dev_plan_out{};
     out.n_items = t.n_items;
     out.n_chunks = static_cast<uint32_t>(t.chunk.size() - 1);
+    out.level_item = t.level_item;
+    out.level_chunk = t.level_chunk;
     if (!(err = alloc(&out.info, t.info.size())).empty() || !(err = alloc(&out.ord, npos)).empty() ||
         !(err = alloc(&out.ptr, npos + 1)).empty() || !(err = alloc(&out.chunk, t.chunk.size())).empty())
         return err;
@@ -637,9 +643,7 @@ bool device_prep_applies(bool fp16, uint32_t n_rounds) {
     if (fp16 || n_rounds == 0) return false;
     if (const char* e = std::getenv("APXB_HOST_PREP"))
         if (*e && *e != '0') return false;
-    if (const char* e = std::getenv("APXB_SEG_LEVEL_ROWS"))   // the serial segment is built on the host
-        if (std::atoi(e) > 0) return false;
-    return kSegLevelRows == 0;
+    return true;
 }
 
 std::string prepare_factor_device(apxb_factor* f, uint32_t n, const uint32_t* colptr, const uint32_t* rowidx,
@@ -784,6 +788,8 @@ std::string prepare_factor_device(apxb_factor* f, uint32_t n, const uint32_t* co
         f->chunk[dir] = o.chunk; f->n_chunks[dir] = o.n_chunks;
         sweep_plan& pl = dir == 0 ? h.fwd_plan : h.bck_plan;
         pl.n_items = o.n_items;
+        pl.level_item = std::move(o.level_item);
+        pl.level_chunk = std::move(o.level_chunk);
     }
     // ---- what stays: the canonical arrays (batch plans, host copies on demand), sizes, counts
     unsigned long long st[3] = {0, 0, 0};
@@ -794,6 +800,7 @@ std::string prepare_factor_device(apxb_factor* f, uint32_t n, const uint32_t* co
     h.dropped = st[1];
     h.dropped_flush = st[2];
     h.fwd_levels = h.bck_levels = n_levels;
+    h.level_bound = lb;
     h.perm.assign(perm, perm + n);
     if (bad[1]) return "perm is not a permutation of [0, n)";
     auto& d = f->dev;

@@ -56,25 +56,6 @@ std::vector<uint32_t> column_ranges(const P* ptr, uint32_t cols, unsigned T) {
 // Plan of one direction (see sweep_plan). level[r] = level of row r in this
 // direction; (ptr, idx, val) = the canonical arrays of the direction (forward:
 // CSR(L11), diagonal last; backward: CSC(L11), diagonal first).
-// APXB_SEG_LEVEL_ROWS overrides kSegLevelRows (0 disables the serial segment).
-uint32_t seg_level_rows_setting() {
-    const char* e = std::getenv("APXB_SEG_LEVEL_ROWS");
-    return e ? static_cast<uint32_t>(std::atoi(e)) : kSegLevelRows;
-}
-
-// Appends row r's entries re-laid (off-diagonals in the reference order, the
-// diagonal last) to (oi, ov).
-void relay_row(uint32_t r, bool forward, const std::vector<uint32_t>& ptr, const plan_vec<uint32_t>& idx,
-               const plan_vec<float>& val, std::vector<uint32_t>& oi, std::vector<float>& ov) {
-    const uint32_t b = ptr[r], en = ptr[r + 1];
-    const uint32_t d = forward ? en - 1 : b;
-    for (uint32_t p = b; p < en; ++p) {
-        if (p == d) continue;
-        oi.push_back(idx[p]); ov.push_back(val[p]);
-    }
-    oi.push_back(idx[d]); ov.push_back(val[d]);
-}
-
 // Rows grouped by (level, class): levels ascending, classes 0..n_cls-1, rows
 // ascending inside a group -- one stable counting sort. cls[r] == n_cls leaves
 // row r out. start[l * n_cls + c] is where group (l, c) begins in rows.
@@ -92,67 +73,24 @@ void group_rows(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels,
 }
 
 // val16 (fp16 storage, nullable): binary16 values beside val, re-laid the
-// same way into plan.val16; such plans have no serial segment.
+// same way into plan.val16.
 void build_plan(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels, const std::vector<uint32_t>& bits,
                 const std::vector<uint32_t>& ptr, const plan_vec<uint32_t>& idx, const plan_vec<float>& val,
-                bool forward, bool contiguous, sweep_plan& plan, const plan_vec<uint16_t>* val16 = nullptr) {
-    if (val16) contiguous = false;
+                bool forward, sweep_plan& plan, const plan_vec<uint16_t>* val16 = nullptr) {
     plan = sweep_plan{};
-    // Serial segment: the trailing run (forward order) of small levels.
-    int32_t seg_from = n_levels;   // in this direction's level numbering: forward [seg_from, n), backward [0, seg_to)
-    int32_t seg_to = 0;
-    const uint32_t seg_rows_max = seg_level_rows_setting();
-    if (contiguous && seg_rows_max > 0) {
-        std::vector<std::vector<uint32_t>> by_level(static_cast<size_t>(n_levels));
-        for (uint32_t r = 0; r < m; ++r) by_level[level[r]].push_back(r);
-        uint32_t rows = 0;
-        int32_t nseg = 0;
-        for (int32_t k = 0; k < n_levels; ++k) {            // k-th level from the forward end
-            const int32_t l = forward ? n_levels - 1 - k : k;
-            const uint32_t c = static_cast<uint32_t>(by_level[l].size());
-            if (c > seg_rows_max || rows + c > kSegMaxRows) break;
-            rows += c;
-            ++nseg;
-        }
-        if (nseg >= static_cast<int32_t>(kSegMinLevels)) {
-            if (forward) seg_from = n_levels - nseg;
-            else seg_to = nseg;
-        }
-        auto in_seg = [&](int32_t l) { return forward ? l >= seg_from : l < seg_to; };
-        if (seg_from < n_levels || seg_to > 0) {
-            plan.seg_first = m;
-            plan.seg_ptr.push_back(0);
-            for (int32_t l = 0; l < n_levels; ++l) {
-                if (!in_seg(l)) continue;
-                const auto& lr = by_level[l];
-                const uint32_t thin = lr.empty() ? 0u : (bits[lr[0] >> 5] >> (lr[0] & 31)) & 1u;
-                plan.seg_lvl.push_back(static_cast<uint32_t>(plan.seg_row.size()) | (thin << 31));
-                for (uint32_t r : lr) {
-                    plan.seg_row.push_back(r);
-                    plan.seg_first = std::min(plan.seg_first, r);
-                    relay_row(r, forward, ptr, idx, val, plan.seg_idx, plan.seg_val);
-                    plan.seg_ptr.push_back(static_cast<uint32_t>(plan.seg_idx.size()));
-                }
-            }
-            plan.seg_levels = static_cast<uint32_t>(plan.seg_lvl.size());
-            plan.seg_lvl.push_back(static_cast<uint32_t>(plan.seg_row.size()));
-            plan.seg_rows = static_cast<uint32_t>(plan.seg_row.size());
-        }
-    }
-    auto in_seg = [&](int32_t l) { return forward ? l >= seg_from : l < seg_to; };
     // items: (level, G) groups, G = 32, 16, 8, 4, 1 (classes 0..4), cut into 32/G rows
     constexpr uint32_t kCls = 5;
     std::vector<uint8_t> cls(m);
     std::vector<uint32_t> first_row(static_cast<size_t>(n_levels), kNoRow);   // a level's smallest row (its thin bit)
     for (uint32_t r = 0; r < m; ++r) {
         const uint32_t g = group_width(ptr[r + 1] - ptr[r] - 1);
-        cls[r] = in_seg(level[r]) ? kCls : static_cast<uint8_t>(g == 1 ? 4 : 5 - __builtin_ctz(g));
+        cls[r] = static_cast<uint8_t>(g == 1 ? 4 : 5 - __builtin_ctz(g));
         if (first_row[level[r]] == kNoRow) first_row[level[r]] = r;
     }
     std::vector<uint32_t> item_rows, start;
     group_rows(m, level, n_levels, cls, kCls, item_rows, start);
     for (int32_t l = 0; l < n_levels; ++l) {
-        if (in_seg(l) || first_row[l] == kNoRow) continue;
+        if (first_row[l] == kNoRow) continue;
         const uint32_t thin = (bits[first_row[l] >> 5] >> (first_row[l] & 31)) & 1u;
         for (uint32_t c = 0; c < kCls; ++c) {
             const size_t key = static_cast<size_t>(l) * kCls + c;
@@ -205,6 +143,7 @@ void build_plan(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels,
     });
     plan.ptr[npos] = total;
     chunk_plan(plan);
+    index_levels(plan, n_levels);
 }
 
 // Plan invariants the kernels rely on (checked at every setup): every row is
@@ -232,22 +171,6 @@ std::string check_plan(uint32_t m, const std::vector<int32_t>& level, const swee
         }
         if (l < prev) return "plan items out of level order";
         prev = l;
-    }
-    if (pl.seg_rows) {
-        if (pl.seg_first + pl.seg_rows != m) return "serial segment is not a suffix";
-        for (uint32_t i = 0; i < pl.seg_rows; ++i) {
-            const uint32_t r = pl.seg_row[i];
-            if (r < pl.seg_first || r >= m || seen[r]) return "bad segment row";
-            seen[r] = 1;
-            if (pl.seg_ptr[i + 1] <= pl.seg_ptr[i] || pl.seg_idx[pl.seg_ptr[i + 1] - 1] != r)
-                return "segment diagonal misplaced";
-        }
-        for (uint32_t l = 0; l < pl.seg_levels; ++l) {
-            const uint32_t lo = pl.seg_lvl[l] & 0x7fffffffu, hi = pl.seg_lvl[l + 1] & 0x7fffffffu;
-            if (hi < lo) return "bad segment level";
-            for (uint32_t i = lo; i < hi; ++i)
-                if (level[pl.seg_row[i]] != level[pl.seg_row[lo]]) return "segment level mixes levels";
-        }
     }
     for (uint32_t r = 0; r < m; ++r)
         if (!seen[r]) return "plan misses row " + std::to_string(r);
@@ -368,6 +291,7 @@ void build_batch_plan(const prepared_factor& h, int dir, uint32_t col_lanes, swe
     });
     plan.ptr[npos] = total;
     chunk_plan(plan);
+    index_levels(plan, n_levels);
 }
 
 void chunk_plan(sweep_plan& p) {
@@ -381,6 +305,35 @@ void chunk_plan(sweep_plan& p) {
         c = e;
     }
     p.chunk.push_back(p.n_items);
+}
+
+void index_levels(sweep_plan& p, int32_t n_levels) {
+    p.level_item.assign(static_cast<size_t>(n_levels) + 1, p.n_items);
+    p.level_chunk.assign(static_cast<size_t>(n_levels) + 1, static_cast<uint32_t>(p.chunk.size() - 1));
+    for (uint32_t c = p.n_items; c-- > 0;) p.level_item[p.item_level[c]] = c;
+    for (uint32_t q = static_cast<uint32_t>(p.chunk.size()) - 1; q-- > 0;) p.level_chunk[p.item_level[p.chunk[q]]] = q;
+    for (int32_t l = n_levels - 1; l >= 0; --l) {   // a level without rows starts where the next one does
+        p.level_item[l] = std::min(p.level_item[l], p.level_item[l + 1]);
+        p.level_chunk[l] = std::min(p.level_chunk[l], p.level_chunk[l + 1]);
+    }
+}
+
+tail_span choose_tail(const prepared_factor& h, uint32_t max_rows) {
+    tail_span t;
+    if (h.level_bound.empty() || h.tail_level_rows == 0) return t;
+    const auto& lb = h.level_bound;
+    int32_t l = h.fwd_levels;
+    while (l > 0 && lb[l] - lb[l - 1] <= h.tail_level_rows && h.m - lb[l - 1] <= max_rows) --l;
+    if (h.fwd_levels - l < kTailMinLevels) return t;
+    t.level = l;
+    t.first = lb[l];
+    t.rows = h.m - lb[l];
+    return t;
+}
+
+uint32_t tail_level_rows_setting() {
+    const char* e = std::getenv("APXB_SEG_LEVEL_ROWS");
+    return e && *e ? static_cast<uint32_t>(std::max(0, std::atoi(e))) : kTailLevelRows;
 }
 
 std::string check_batch_plan(uint32_t m, const std::vector<int32_t>& level, const sweep_plan& pl, uint32_t col_lanes) {
@@ -640,6 +593,9 @@ std::string prepare_factor(uint32_t n, const uint32_t* colptr, const uint32_t* r
         }
         for (uint32_t c = 0; c < m; ++c) bl[c] = maxd - fl[c];
         out.fwd_levels = out.bck_levels = maxd + 1;
+        out.level_bound.assign(static_cast<size_t>(maxd) + 2, m);   // fl ascends: levels are row ranges
+        for (uint32_t c = m; c-- > 0;) out.level_bound[fl[c]] = c;
+        for (int32_t l = maxd; l >= 0; --l) out.level_bound[l] = std::min(out.level_bound[l], out.level_bound[l + 1]);
         done = true;
     }
     if (!done) {
@@ -668,11 +624,11 @@ std::string prepare_factor(uint32_t n, const uint32_t* colptr, const uint32_t* r
     std::string bad[2];
     run_threads(2, [&](unsigned dir) {
         if (dir == 1) {
-            build_plan(m, bl, out.bck_levels, out.bck_thin_bits, cp, ci, cv, false, done, out.bck_plan,
+            build_plan(m, bl, out.bck_levels, out.bck_thin_bits, cp, ci, cv, false, out.bck_plan,
                        fp16 ? &ch : nullptr);
             bad[1] = check_plan(m, bl, out.bck_plan);
         } else {
-            build_plan(m, fl, out.fwd_levels, out.fwd_thin_bits, out.csr_ptr, out.csr_idx, out.csr_val, true, done,
+            build_plan(m, fl, out.fwd_levels, out.fwd_thin_bits, out.csr_ptr, out.csr_idx, out.csr_val, true,
                        out.fwd_plan, fp16 ? &out.csr_h : nullptr);
             bad[0] = check_plan(m, fl, out.fwd_plan);
         }

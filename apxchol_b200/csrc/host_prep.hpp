@@ -147,15 +147,9 @@ using plan_vec = std::vector<T, uninit_alloc<T>>;
 //    ascending), then the diagonal last, at [ptr[pos], ptr[pos + 1]).
 //  * `info[c]` = count | log2(G) << 8 | thin << 16 (thin: the level uses the
 //    4-way split sum; a level property, so uniform in an item).
-//  * The serial segment (round-as-level factors only): the run of small
-//    levels at the end of the elimination (the forward sweep's last levels,
-//    the backward sweep's first), at most kSegLevelRows rows each. One thread
-//    block solves it level by level through shared memory and __syncthreads,
-//    which is far cheaper per level than a cross-SM dependency hop. Its rows
-//    are the suffix [seg_first, m); `seg_row` lists them in processing order,
-//    `seg_lvl` holds each level's start in that list (seg_levels + 1 words,
-//    bit 31 = thin level), and their entries are re-laid like the items'
-//    (`seg_ptr` per listed row, diagonal last).
+//  * level_item / level_chunk: a level's first item and first claim unit (level
+//    n_levels: their ends). A sweep hands the items of the narrow last levels of
+//    the elimination to a cluster launch (choose_tail; sweep.cu).
 struct sweep_plan {
     uint32_t n_items = 0;
     std::vector<int32_t> item_level;   // level of each item (host side; batch plans)
@@ -166,16 +160,8 @@ struct sweep_plan {
     plan_vec<uint32_t> idx;
     plan_vec<float> val;
     plan_vec<uint16_t> val16;          // fp16 storage: the binary16 values, same layout as val
-    uint32_t seg_first = 0, seg_rows = 0, seg_levels = 0;
-    std::vector<uint32_t> seg_row, seg_lvl, seg_ptr, seg_idx;
-    std::vector<float> seg_val;
+    std::vector<uint32_t> level_item, level_chunk;
 };
-
-// The serial segment is off by default (APXB_SEG_LEVEL_ROWS=<rows> enables it):
-// on the factors measured so far the cross-SM dataflow hop beat it.
-constexpr uint32_t kSegLevelRows = 0;    // a level joins the serial segment when it has <= this many rows
-constexpr uint32_t kSegMaxRows = 4096;   // segment values stay in shared memory (fp64: 32 KB)
-constexpr uint32_t kSegMinLevels = 8;    // fewer small trailing levels than this: no segment
 
 constexpr uint32_t kNoRow = 0xffffffffu;
 
@@ -198,6 +184,8 @@ struct prepared_factor {
     int32_t fwd_levels = 0, bck_levels = 0;
     std::vector<uint32_t> perm;  // perm[original] = position
     std::vector<int32_t> fwd_level, bck_level;   // level of every row per direction
+    std::vector<uint32_t> level_bound;           // forward level l = rows [l, l + 1) of it (empty: levels are not row ranges)
+    uint32_t tail_level_rows = 0;                // largest level of the cluster tail (0: none)
     sweep_plan fwd_plan, bck_plan;
     // fp16 storage (the reference's cuda_sptrsv default, cuda.h:131-163;
     // cuda_host.h:16-34): column j is stored scaled by 1 / s_j (s_j the
@@ -240,6 +228,22 @@ void build_batch_plan(const prepared_factor& h, int dir, uint32_t col_lanes, swe
 // level, max(1, min(8, items of the level / 4096)) per unit, so large levels
 // take one work-counter claim per several items while every warp stays busy.
 void chunk_plan(sweep_plan& p);
+// Fills level_item and level_chunk from item_level and chunk.
+void index_levels(sweep_plan& p, int32_t n_levels);
+
+// The cluster tail of a factor: the longest run of last levels (row ranges) of
+// at most tail_level_rows rows each and max_rows together; none below
+// kTailMinLevels levels (a launch costs about as much as two levels save).
+struct tail_span {
+    int32_t level = 0;        // its first forward level; backward it is the first fwd_levels - level levels
+    uint32_t first = 0, rows = 0;
+};
+constexpr uint32_t kTailLevelRows = 512;
+constexpr int32_t kTailMinLevels = 4;
+tail_span choose_tail(const prepared_factor& h, uint32_t max_rows);
+// kTailLevelRows, or APXB_SEG_LEVEL_ROWS (0: no tail).
+uint32_t tail_level_rows_setting();
+
 // Invariants of a batch plan (rows once each, items in level order within one
 // level, G >= col_lanes, diagonal last, chunks cover the items).
 std::string check_batch_plan(uint32_t m, const std::vector<int32_t>& level, const sweep_plan& p, uint32_t col_lanes);

@@ -14,6 +14,35 @@ struct sweep_ctl {
     unsigned done;
 };
 
+// The cluster tail of a sweep: the items [item0, item1) of its plan, which solve
+// the rows [first, first + rows) -- the last rows of the elimination, in levels
+// that are row ranges (rows == 0: no tail). The plan's claim units outside the
+// tail are [0, chunk) forward and [chunk, n_chunks) backward.
+struct tail_plan {
+    int cluster = 0;                   // CTAs per cluster
+    uint32_t chunk = 0, item0 = 0, item1 = 0, first = 0, rows = 0;
+};
+template <class T>
+struct tail_args {
+    const uint32_t* info; const uint32_t* ord; const uint32_t* ptr; const uint32_t* idx;
+    const float* val;
+    const uint16_t* val16; const float* diag16; const double* scale2;   // fp16 storage (see sweep_args)
+    uint32_t item0, item1, first, rows;
+    int k;                             // columns per row of the vectors
+    int wide;                          // the plan is a batch plan (k <= 4), else a factor plan
+    const T* in; const double* in64; const double* rhs_sub;
+    T* out; T* reset; T* copy_out;
+    dev_error* err; const int* skip;
+    unsigned long long budget_ns;
+};
+constexpr uint32_t kTailSmem = 200 * 1024;   // the solution copy of a CTA
+// fp32 tails hold up to 4 columns a row; the same rows whatever k is, since a
+// factor plan's rows are summed by other lanes there than in the dataflow launch
+// and a column's result should not depend on the columns beside it.
+constexpr uint32_t kTailRows32 = kTailSmem / (4 * sizeof(float));
+// CTAs of a tail cluster on the current device (16, else 8; 0: no cluster fits).
+int tail_cluster_size();
+
 // One sync-free sweep over a prepared direction of the factor (forward:
 // L y = x over CSR(L11); backward: L^T z = y over CSC(L11)), driven by the
 // direction's plan (host_prep.hpp, sweep_plan).
@@ -29,13 +58,6 @@ struct sweep_args {
     const uint32_t* ptr;              // per position: entry range in idx / val (diagonal last)
     const uint32_t* idx;
     const float* val;
-    // serial segment (see sweep_plan): rows [seg_first, seg_first + seg_rows)
-    uint32_t seg_first, seg_rows, seg_levels;
-    const uint32_t* seg_row;
-    const uint32_t* seg_lvl;
-    const uint32_t* seg_ptr;
-    const uint32_t* seg_idx;
-    const float* seg_val;
     const T* in;                      // right-hand side, row-major [row][k]
     const double* rhs_sub;            // nullable: device scalar(s) subtracted from every rhs
     T* out;                           // tracked solution [row][k]
@@ -57,6 +79,7 @@ struct sweep_args {
     const uint16_t* val16;
     const float* diag16;
     const double* in_scale2;
+    const tail_plan* tail;            // nullable: the narrow last levels go to a cluster launch (host side)
 };
 
 // fp64 sweep reproducing the reference CPU arithmetic (exact sum order).

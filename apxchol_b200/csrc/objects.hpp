@@ -76,6 +76,7 @@ struct apxb_engine {
     int vec_grid = 592;
     int center_k = 10;
     int sweep_grid = 0;                   // 0 = resident grid
+    int tail_cluster = 0;                 // CTAs of a tail cluster (0: no cluster launches)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // staging for host-pointer entry points
     double* d_stage_a = nullptr; double* d_stage_b = nullptr; size_t stage_n = 0;
@@ -175,9 +176,7 @@ struct apxb_factor {
     double* inv_scale2 = nullptr;                      // fp16 factors: per-row (1 / s)^2, fp64
     uint32_t* chunk[2] = {nullptr, nullptr};           // claim units (host_prep.hpp, chunk_plan)
     uint32_t n_chunks[2] = {0, 0};
-    uint32_t *seg_row[2] = {nullptr, nullptr}, *seg_lvl[2] = {nullptr, nullptr};
-    uint32_t *seg_ptr[2] = {nullptr, nullptr}, *seg_idx[2] = {nullptr, nullptr};
-    float* seg_val[2] = {nullptr, nullptr};
+    apxb::tail_plan tail[2][2];                        // cluster tails per direction: fp64 sweeps, fp32 sweeps
     // Factors prepared on the device (devprep.cu): the canonical arrays stay
     // there for batch plans; h then holds sizes and counts only, and its
     // arrays are filled on demand (factor_host_arrays).
@@ -273,19 +272,22 @@ inline void plan_args(const apxb_factor* f, int dir, apxb::sweep_args<T>& a) {
     a.val16 = f->val16[dir];
     a.diag16 = f->diag16;
     a.in_scale2 = nullptr;   // set for the backward of an fp16 factor by its caller
-    a.seg_first = pl.seg_first;
-    a.seg_rows = pl.seg_rows;
-    a.seg_levels = pl.seg_levels;
-    a.seg_row = f->seg_row[dir];
-    a.seg_lvl = f->seg_lvl[dir];
-    a.seg_ptr = f->seg_ptr[dir];
-    a.seg_idx = f->seg_idx[dir];
-    a.seg_val = f->seg_val[dir];
     a.chunk = f->chunk[dir];
     a.n_chunks = f->n_chunks[dir];
 }
 
+// The tail launch of direction dir of the fp64 or the fp32 sweeps, or null.
+inline const apxb::tail_plan* tail_of(const apxb_factor* f, int dir, bool fp32) {
+    const apxb::tail_plan& t = f->tail[dir][fp32 ? 1 : 0];
+    return t.rows ? &t : nullptr;
+}
+
 namespace apxb {
+// The cluster tail of a plan of factor f in direction dir when a CTA holds
+// max_rows rows; the plan by its levels' first items and claim units.
+tail_plan plan_tail(const apxb_factor* f, int dir, uint32_t max_rows, const std::vector<uint32_t>& level_item,
+                    const std::vector<uint32_t>& level_chunk);
+
 // Device preparation (devprep.cu): the host preparation's arrays, byte for
 // byte, built by kernels. Applies to fp32/fp64 storage with round sizes.
 bool device_prep_applies(bool fp16, uint32_t n_rounds);
@@ -302,6 +304,7 @@ struct dev_plan_out {
     uint64_t n_entries = 0;
     uint32_t *info = nullptr, *ord = nullptr, *ptr = nullptr, *idx = nullptr, *chunk = nullptr;
     float* val = nullptr;
+    std::vector<uint32_t> level_item, level_chunk;   // as sweep_plan's
 };
 std::string batch_plan_device(const apxb_factor* f, int dir, uint32_t col_lanes,
                               const std::function<std::string(void**, size_t)>& alloc_bytes, dev_plan_out& out,

@@ -4,10 +4,10 @@
 // omp_sptrsv::solve_levelset, include/apxchol/solver/sptrsv/omp.h:1094-1119).
 //
 // Design (B200):
-//  * A sweep is a dataflow launch plus, for factors whose elimination ends in
-//    a long run of tiny rounds, a serial-segment launch (one block, shared
-//    memory, __syncthreads per level; forward: after the dataflow, backward:
-//    before it). The dataflow grid's warps work off the direction's plan
+//  * A sweep is a dataflow launch plus, for the run of narrow levels that the
+//    elimination ends in, a cluster-tail launch (one thread-block cluster,
+//    solved rows in distributed shared memory; forward: after the dataflow,
+//    backward: before it). The dataflow grid's warps work off the plan
 //    (host_prep.hpp, sweep_plan): work items of up to 32 rows
 //    of one level and one lane-group width G, G lanes per row, with the rows'
 //    entries re-laid in processing order. A warp claims items from an atomic
@@ -31,21 +31,21 @@
 //    levels use the 4-way split sum of dot_thin (omp.h:1343-1357), rows of
 //    "fat" levels one serial sum (omp.h:1434-1439), finished by one correctly
 //    rounded subtract and divide (omp.h:1440). With G lanes per row the
-//    products are formed in parallel and the order is replayed through
-//    shuffles: the result is the reference CPU sweep's bytes.
+//    products are formed in parallel and the order is replayed from shared
+//    memory: the result is the reference CPU sweep's bytes.
 //  * fp32 sweep: fp32 values and fp32 fused multiply-add accumulation, each
-//    lane adding its entries in order as they arrive, lane partials combined
-//    by a fixed butterfly (deterministic); k right-hand sides per row
+//    lane adding its entries in order, oldest dependency first, lane partials
+//    combined by a fixed butterfly (deterministic); k right-hand sides per row
 //    interleaved [row][k]: each factor entry is read once for all k.
-//  * Rows are consumed progressively: in the fp64 sweep the reference's sum
-//    order is advanced step by step as operands arrive, so most of a row's
-//    arithmetic is done before its last dependency lands.
+//  * Rows are consumed progressively in the fp64 sweep: the reference's sum
+//    order is advanced as operands arrive, so most of a row's arithmetic is
+//    done before its last dependency lands.
 //  * fp16 factor storage (the reference's GPU default, cuda.h:131-163): the
 //    fp32 sweep reads binary16 weights of the column-scaled factor, widened
 //    exactly to fp32, a per-row fp32 diagonal, and (backward) its right-hand
 //    side times the fp64 inv_scale^2 (cuda_dataflow.cu:395), 6 instead of 8
 //    bytes per stored entry.
-#include <cstdlib>
+#include <algorithm>
 #include <cuda_fp16.h>
 
 #include "kernels.cuh"
@@ -105,50 +105,58 @@ __device__ __forceinline__ double dadd4(double a, double b, double c, double d) 
     return __dadd_rn(__dadd_rn(a, b), __dadd_rn(c, d));
 }
 
-// ---------------------------------------------------------------------------
-// Exact-order accumulation for a G-lane group (G = 2^LG = 4..32). Lane u of
-// the group holds the product of entry t = t0 + u of the current step.
-// thin: chain c (entries t = c mod 4, t < gend) accumulates in lane c in entry
-// order; the step holding gend (when the row has a tail, gend < len) then
-// combines the chains as (s0 + s1) + (s2 + s3) and adds the <= 3 tail entries
-// in order. fat: lane 0 adds every entry in order. Steps are consumed in
-// order, each as soon as all of its operands are ready, so most of a row's
-// arithmetic is done before its last dependency arrives.
-struct exact_state {
-    double s = 0.0, sum = 0.0;
-    bool combined = false;
+// a / d correctly rounded for a divisor known before a, in two dependent
+// operations: with 1 / d = h + l (l the rounded remainder of h = RN(1 / d), so
+// the pair is within 2^-104), RN(a h + RN(a l)) differs from a / d by less than
+// 2^-103 of it before its one rounding. d is an fp32 value: a / d lies at least
+// 2^-79 of itself away from every midpoint of two doubles (a - m d is a nonzero
+// whole multiple of the unit of the 54-bit m times the 24-bit d; it is not zero
+// since m d has more than 53 bits), so the rounding is that of a / d. Operands
+// near overflow or underflow divide. fp64 operations take about 40 cycles each
+// on the row's critical path here (a divide about nine of them).
+struct recip64 {
+    double d, h, l;
+    unsigned span;   // exponents of a that take the short way: [123, 123 + span)
+    __device__ __forceinline__ double quotient(double a) const {
+        double q = __fma_rn(a, h, __dmul_rn(a, l));
+        if (((static_cast<unsigned>(__double2hiint(a)) >> 20) & 0x7ffu) - 123u >= span) q = __ddiv_rn(a, d);
+        return q;
+    }
 };
+__device__ __forceinline__ recip64 recip_of(double d) {
+    const double h = __drcp_rn(d);
+    const unsigned ed = (static_cast<unsigned>(__double2hiint(d)) >> 20) & 0x7ffu;
+    return {d, h, __dmul_rn(__fma_rn(-d, h, 1.0), h), ed - (1023u - 120u) < 240u ? 1750u : 0u};
+}
 
+// ---------------------------------------------------------------------------
+// Exact-order accumulation for a G-lane group (G = 2^LG = 4..32). The products
+// of a batch of kBatch steps of G entries lie in shared memory (pr: entry t of
+// the row's batch from step jb on at 32 * (t / G - jb) + t % G). thin: chain c
+// (entries t = c mod 4, t < gend) accumulates in lane c in entry order; fat:
+// lane 0 adds every entry in order. The leading entries that have arrived are
+// consumed, so most of a row's arithmetic is done before its last dependency
+// arrives. The chain of dependent additions bounds this, so the products come
+// from shared memory, where the loads run ahead of the chain.
 template <unsigned LG>
-__device__ __forceinline__ void exact_step(bool thin, bool consume, unsigned u, uint32_t t0, uint32_t len,
-                                           uint32_t gend, double pk, exact_state& e) {
-    constexpr unsigned G = 1u << LG;
-    if (thin) {
-        const unsigned c = u & 3u;
+__device__ __forceinline__ unsigned prod_at(uint32_t t, uint32_t jb) {
+    return 32u * ((t >> LG) - jb) + (t & ((1u << LG) - 1u));
+}
+
+// Lane u's entries u, u + W, ... (W chains) from `at` while at + W <= upto.
+template <unsigned LG, unsigned W>
+__device__ __forceinline__ void chain_to(const double* pr, uint32_t jb, unsigned u, uint32_t upto, uint32_t& at, double& sum) {
+    while (at + 8u * W <= upto) {
+        double v[8];
 #pragma unroll
-        for (unsigned i = 0; i < G / 4; ++i) {
-            const double v = __shfl_sync(kFull, pk, static_cast<int>(c + 4u * i), static_cast<int>(G));
-            if (consume && u < 4 && t0 + c + 4u * i < gend) e.s = __dadd_rn(e.s, v);
-        }
-        const bool tail = consume && !e.combined && gend < len && (gend >> LG) == (t0 >> LG);
-        if (__any_sync(kFull, tail)) {
-            const double s1 = __shfl_sync(kFull, e.s, 1, static_cast<int>(G));
-            const double s2 = __shfl_sync(kFull, e.s, 2, static_cast<int>(G));
-            const double s3 = __shfl_sync(kFull, e.s, 3, static_cast<int>(G));
-            if (tail && u == 0) e.sum = dadd4(e.s, s1, s2, s3);
+        for (unsigned i = 0; i < 8; ++i) v[i] = pr[prod_at<LG>(at + W * i + u, jb)];
 #pragma unroll
-            for (unsigned i = 0; i < 3; ++i) {
-                const double v = __shfl_sync(kFull, pk, static_cast<int>((gend + i) & (G - 1u)), static_cast<int>(G));
-                if (tail && u == 0 && gend + i < len) e.sum = __dadd_rn(e.sum, v);
-            }
-            if (tail) e.combined = true;
-        }
-    } else {
-#pragma unroll
-        for (unsigned i = 0; i < G; ++i) {
-            const double v = __shfl_sync(kFull, pk, static_cast<int>(i), static_cast<int>(G));
-            if (consume && u == 0 && t0 + i < len) e.s = __dadd_rn(e.s, v);
-        }
+        for (unsigned i = 0; i < 8; ++i) sum = __dadd_rn(sum, v[i]);
+        at += 8u * W;
+    }
+    while (at + W <= upto) {
+        sum = __dadd_rn(sum, pr[prod_at<LG>(at + u, jb)]);
+        at += W;
     }
 }
 
@@ -178,6 +186,7 @@ __device__ __forceinline__ void load_desc(const sweep_args<T>& a, unsigned c, st
 // Lane view of an item after stage D: the lane's group, its row, and its range.
 struct lane_view {
     unsigned c, lg, G, u, gid;
+    unsigned rows;          // rows of the item
     bool valid, thin;
     uint32_t row, q, len;   // off-diagonals at [q, q + len); diagonal at q + len
 };
@@ -186,6 +195,7 @@ __device__ __forceinline__ lane_view view_of(const stage_desc& d) {
     const unsigned lane = threadIdx.x & 31u;
     lane_view v;
     v.c = d.c;
+    v.rows = d.info & 0xffu;
     v.lg = (d.info >> 8) & 0xffu;
     v.G = 1u << v.lg;
     v.u = lane & (v.G - 1u);
@@ -249,7 +259,7 @@ struct chunk_claim {
 // Stage L data of one item (fp64).
 struct stage_data64 {
     lane_view v;
-    double rhs, d;
+    double rhs, d;   // of the group's first lane
     uint32_t jj[kBatch];
     float ww[kBatch];
 };
@@ -270,137 +280,197 @@ __device__ __forceinline__ void load_data64(const sweep_args<double>& a, const s
     }
 }
 
-// Group rows (G = 2^LG lanes per row): batches of kBatch steps; inside a
-// batch the steps are consumed in order as their operands arrive.
+// Where the rows' operands are read and how a warp waits for them.
+struct far_src64 {
+    const sweep_args<double>& a;
+    int where;
+    bool back;                      // the newest dependency comes first (backward plans), else last
+    idle_clock clk;
+    __device__ __forceinline__ void load(bool on, uint32_t j, double& y) const { ld_if(on, a.out + j, y); }
+    __device__ __forceinline__ bool idle(uint32_t row) { return clk.idle(a.err, a.budget_ns, where, row); }
+    __device__ __forceinline__ void progress() { clk.spins = 0; }
+};
+
+// A lane waits on its newest pending operand alone, kLight polls at a time
+// between passes over all of them: what it waits for last arrives last, and
+// every poll of every waiting warp is a load that the working warps' loads
+// queue behind.
+constexpr int kLight = 4;
+
+// k of the newest pending operand (bit k of pend), and its row and weight.
+__device__ __forceinline__ int newest_of(unsigned pend, bool back) {
+    return back ? __ffs(pend) - 1 : 31 - __clz(pend);
+}
+template <class V, int B>
+__device__ __forceinline__ V pick(const V (&v)[B], int k) {
+    V r = v[0];
+#pragma unroll
+    for (int i = 1; i < B; ++i) r = k == i ? v[i] : r;
+    return r;
+}
+
+// Group rows (G = 2^LG lanes per row): batches of kBatch steps. A lane puts the
+// product of an operand that has arrived into shared memory (prod: 32 doubles a
+// step, the warp's own), and every group consumes its leading entries.
 template <unsigned LG>
-__device__ __forceinline__ bool run_group64(const sweep_args<double>& a, stage_data64& s, int where,
-                                            double& total) {
+__device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, double* prod, double& total) {
     constexpr unsigned G = 1u << LG;
     const lane_view& v = s.v;
-    const unsigned gmask = G == 32 ? kFull : (((1u << G) - 1u) << (v.gid * G));
-    const uint32_t J = (v.len + G - 1u) >> LG;
-    const uint32_t Jmax = __reduce_max_sync(kFull, J);
-    const uint32_t gend = v.thin ? (v.len & ~3u) : 0u;
-    exact_state e;
-    idle_clock clk;
+    const unsigned lane = threadIdx.x & 31u;
+    const double* pr = prod + G * v.gid;
+    const uint32_t Jmax = __reduce_max_sync(kFull, (v.len + G - 1u) >> LG);
+    const uint32_t gend = v.thin ? (v.len & ~3u) : v.len;   // entries the chains take
+    double sum = 0.0;
+    uint32_t at = 0;
     for (uint32_t jb = 0; jb < Jmax; jb += kBatch) {
         if (jb > 0) {
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
                 const uint32_t t = ((jb + k) << LG) + v.u;
-                if (t < v.len) { s.jj[k] = __ldg(a.idx + v.q + t); s.ww[k] = __ldg(a.val + v.q + t); }
+                if (t < v.len) { s.jj[k] = __ldg(src.a.idx + v.q + t); s.ww[k] = __ldg(src.a.val + v.q + t); }
             }
+            __syncwarp();   // the last batch's products have been read
         }
-        const uint32_t nsteps = J > jb ? min(static_cast<uint32_t>(kBatch), J - jb) : 0u;
-        double p[kBatch];
-        unsigned rdy = 0;   // bit k: entry of step k absent or its product is in p[k]
+        unsigned pend = 0;   // bit k: the operand of step k is still to come
+        double y[kBatch];
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
-            const uint32_t t = ((jb + k) << LG) + v.u;
-            p[k] = 0.0;
-            if (t < v.len) p[k] = ld_relaxed(a.out + s.jj[k]);
+            const bool on = ((jb + k) << LG) + v.u < v.len;
+            y[k] = sent_of(0.0);
+            src.load(on, s.jj[k], y[k]);
+            pend |= on ? 1u << k : 0u;
         }
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            const uint32_t t = ((jb + k) << LG) + v.u;
-            if (t >= v.len) rdy |= 1u << k;
-            else if (!is_sent(p[k])) { p[k] = __dmul_rn(static_cast<double>(s.ww[k]), p[k]); rdy |= 1u << k; }
-        }
-        uint32_t kpos = 0;
         for (;;) {
-            bool progressed = false;
 #pragma unroll
-            for (int k = 0; k < kBatch; ++k) {
-                const unsigned bal = __ballot_sync(kFull, (rdy >> k) & 1u);
-                const bool consume = kpos == static_cast<uint32_t>(k) && static_cast<uint32_t>(k) < nsteps &&
-                                     (bal & gmask) == gmask;
-                if (__any_sync(kFull, consume)) {
-                    exact_step<LG>(v.thin, consume, v.u, (jb + k) << LG, v.len, gend, p[k], e);
-                    progressed = true;
+            for (int k = 0; k < kBatch; ++k)
+                if (((pend >> k) & 1u) && !is_sent(y[k])) {
+                    prod[32 * k + lane] = __dmul_rn(static_cast<double>(s.ww[k]), y[k]);
+                    pend &= ~(1u << k);
                 }
-                if (consume) ++kpos;
+            bool open;
+            for (int light = 0;; ++light) {
+                // consume the entries before the group's first pending one
+                __syncwarp();
+                const unsigned any = __reduce_or_sync(kFull, pend);
+                open = any != 0;
+                const uint32_t st = open ? static_cast<uint32_t>(__ffs(any)) - 1u : kBatch;   // leading complete steps
+                const unsigned miss = __ballot_sync(kFull, open && ((pend >> st) & 1u));
+                const unsigned mine = G == 32 ? miss : (miss >> (v.gid * G)) & ((1u << (G & 31u)) - 1u);
+                const uint32_t upto = min(gend, ((jb + st) << LG) + (mine ? static_cast<uint32_t>(__ffs(mine)) - 1u
+                                                                          : (open ? G : 0u)));
+                const uint32_t from = at;
+                if (v.thin) {
+                    if (v.u < 4) chain_to<LG, 4>(pr, jb, v.u, upto, at, sum);
+                } else if (v.u == 0) {
+                    chain_to<LG, 1>(pr, jb, 0, upto, at, sum);
+                }
+                if (!open) break;
+                if (__any_sync(kFull, at != from)) src.progress();
+                else if (src.idle(v.row)) return false;
+                if (light == kLight) break;
+                const int kn = newest_of(pend, src.back);
+                double w = sent_of(0.0);
+                src.load(pend != 0, pick(s.jj, kn), w);
+                if (pend && !is_sent(w)) {
+                    prod[32 * kn + lane] = __dmul_rn(static_cast<double>(pick(s.ww, kn)), w);
+                    pend &= ~(1u << kn);
+                }
             }
-            if (__all_sync(kFull, kpos >= nsteps)) break;
-            if (progressed) clk.spins = 0;
-            else if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
+            if (!open) break;
 #pragma unroll
-            for (int k = 0; k < kBatch; ++k) {
-                if (!((rdy >> k) & 1u)) {
-                    const double y = ld_relaxed(a.out + s.jj[k]);
-                    if (!is_sent(y)) { p[k] = __dmul_rn(static_cast<double>(s.ww[k]), y); rdy |= 1u << k; }
-                }
-            }
+            for (int k = 0; k < kBatch; ++k) src.load((pend >> k) & 1u, s.jj[k], y[k]);
         }
     }
-    const double s1 = __shfl_sync(kFull, e.s, 1, static_cast<int>(G));
-    const double s2 = __shfl_sync(kFull, e.s, 2, static_cast<int>(G));
-    const double s3 = __shfl_sync(kFull, e.s, 3, static_cast<int>(G));
-    total = !v.thin ? e.s : (e.combined ? e.sum : dadd4(e.s, s1, s2, s3));
+    const double s1 = __shfl_sync(kFull, sum, 1, static_cast<int>(G));
+    const double s2 = __shfl_sync(kFull, sum, 2, static_cast<int>(G));
+    const double s3 = __shfl_sync(kFull, sum, 3, static_cast<int>(G));
+    if (v.thin) {   // the chains, then the <= 3 entries after gend (a row's last batch is the warp's)
+        sum = dadd4(sum, s1, s2, s3);
+        const uint32_t jl = Jmax ? ((Jmax - 1u) / kBatch) * kBatch : 0u;
+        if (v.u == 0)
+            for (uint32_t t = gend; t < v.len; ++t) sum = __dadd_rn(sum, pr[prod_at<LG>(t, jl)]);
+    }
+    __syncwarp();   // the products have been read
+    total = sum;
     return true;
 }
 
-// One lane per row (<= kBatch off-diagonals): each lane consumes its entries
-// in order as they arrive, 4-way rotating chains then the serial tail.
-__device__ __forceinline__ bool run_lane64(const sweep_args<double>& a, stage_data64& s, int where, double& total) {
+// The sum of a row of n <= kBatch products in the reference's order: chains
+// 0..3 over the entries before gend, the rest in order. nmax: the warp's
+// longest row (fp64 additions cost their latency also where they are masked).
+__device__ __forceinline__ double lane_sum64(const double (&p)[kBatch], uint32_t n, uint32_t nmax, uint32_t gend) {
+    double sum = 0.0;
+    if (__any_sync(kFull, gend != 0)) {
+        double c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            c[k] = __dadd_rn(0.0, p[k]);
+            const double c8 = __dadd_rn(c[k], p[4 + k]);
+            c[k] = gend == 8 ? c8 : c[k];
+        }
+        const double q = dadd4(c[0], c[1], c[2], c[3]);
+        sum = gend ? q : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+        if (static_cast<uint32_t>(k) >= nmax) break;
+        if (static_cast<uint32_t>(k) >= gend && static_cast<uint32_t>(k) < n) sum = __dadd_rn(sum, p[k]);
+    }
+    return sum;
+}
+
+// One lane per row (<= kBatch off-diagonals): all operands, then the sum in
+// straight line.
+__device__ __forceinline__ bool run_lane64(far_src64& src, stage_data64& s, double& total) {
     const lane_view& v = s.v;
     const uint32_t n = v.len;   // <= kBatch for these rows
-    const uint32_t gend = v.thin ? (n & ~3u) : 0u;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, sum = 0.0;
-    bool combined = false;
-    double yv[kBatch];
+    double y[kBatch];
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k)
-        if (static_cast<uint32_t>(k) < n) yv[k] = ld_relaxed(a.out + s.jj[k]);
-    uint32_t kpos = 0;
-    idle_clock clk;
-    for (;;) {
-        const uint32_t before = kpos;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            if (kpos == static_cast<uint32_t>(k) && kpos < n && !is_sent(yv[k])) {
-                const double pr = __dmul_rn(static_cast<double>(s.ww[k]), yv[k]);
-                if (kpos < gend) {
-                    const double w = __dadd_rn(s0, pr);
-                    s0 = s1; s1 = s2; s2 = s3; s3 = w;
-                } else {
-                    if (!combined) { sum = dadd4(s0, s1, s2, s3); combined = true; }
-                    sum = __dadd_rn(sum, pr);
-                }
-                ++kpos;
-            }
-        }
-        if (__all_sync(kFull, kpos >= n)) break;
-        if (__any_sync(kFull, kpos != before)) clk.spins = 0;
-        else if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k)
-            if (static_cast<uint32_t>(k) >= kpos && static_cast<uint32_t>(k) < n && is_sent(yv[k]))
-                yv[k] = ld_relaxed(a.out + s.jj[k]);
+    for (int k = 0; k < kBatch; ++k) {
+        y[k] = sent_of(0.0);
+        src.load(static_cast<uint32_t>(k) < n, s.jj[k], y[k]);
     }
-    total = combined ? sum : dadd4(s0, s1, s2, s3);
+    for (;;) {
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) open |= static_cast<uint32_t>(k) < n && is_sent(y[k]);
+        if (!__any_sync(kFull, open)) break;
+        if (src.idle(v.row)) return false;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) src.load(static_cast<uint32_t>(k) < n && is_sent(y[k]), s.jj[k], y[k]);
+    }
+    double p[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) p[k] = __dmul_rn(static_cast<double>(s.ww[k]), y[k]);
+    total = lane_sum64(p, n, __reduce_max_sync(kFull, n), v.thin ? (n & ~3u) : 0u);
     return true;
+}
+
+// The off-diagonal sums of one item's rows in the reference's order. Returns
+// false when the warp must drain.
+__device__ __forceinline__ bool run_rows64(far_src64& src, stage_data64& s, double* prod, double& total) {
+    switch (s.v.lg) {
+        case 0: return run_lane64(src, s, total);
+        case 2: return run_group64<2>(src, s, prod, total);
+        case 3: return run_group64<3>(src, s, prod, total);
+        case 4: return run_group64<4>(src, s, prod, total);
+        default: return run_group64<5>(src, s, prod, total);
+    }
 }
 
 // Run one item: wait for its operands, replay the reference's sum order, store.
 // Returns false when the warp must drain.
 template <int DIR>
-__device__ __forceinline__ bool run64(const sweep_args<double>& a, stage_data64& s) {
+__device__ __forceinline__ bool run64(const sweep_args<double>& a, stage_data64& s, double* prod) {
     const lane_view& v = s.v;
-    const int where = DIR == 0 ? kFwdSweep : kBckSweep;
     double total = 0.0;
-    bool ok;
-    switch (v.lg) {
-        case 0: ok = run_lane64(a, s, where, total); break;
-        case 2: ok = run_group64<2>(a, s, where, total); break;
-        case 3: ok = run_group64<3>(a, s, where, total); break;
-        case 4: ok = run_group64<4>(a, s, where, total); break;
-        default: ok = run_group64<5>(a, s, where, total); break;
-    }
-    if (!ok) return false;
+    const recip64 inv = recip_of(s.d);
+    far_src64 src{a, DIR == 0 ? kFwdSweep : kBckSweep, DIR == 1, {}};
+    if (!run_rows64(src, s, prod, total)) return false;
     if (v.valid && v.u == 0) {
         double rhs = s.rhs;
         if (a.rhs_sub) rhs = __dsub_rn(rhs, *a.rhs_sub);
-        const double y = __ddiv_rn(__dsub_rn(rhs, total), s.d);
+        const double y = inv.quotient(__dsub_rn(rhs, total));
         st_relaxed(a.out + v.row, y);
         if (a.copy_out) a.copy_out[v.row] = y;
         // re-arm after the right-hand side was consumed: the backward sweep
@@ -414,7 +484,9 @@ __device__ __forceinline__ bool run64(const sweep_args<double>& a, stage_data64&
 template <int DIR>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_df64(const sweep_args<double> a) {
     if (a.skip && *a.skip) return;
+    __shared__ __align__(16) double prods[kSweepThreads / 32][32 * kBatch];
     const unsigned lane = threadIdx.x & 31u;
+    double* prod = prods[threadIdx.x >> 5];
     chunk_claim cc;
     cc.start(a);
     stage_desc dD;
@@ -430,7 +502,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_df64(const sweep_args<doub
         load_desc(a, cc.next(a), dD);
         if (__shfl_sync(kFull, bad, 0)) break;
         if (lane == 0) bad = ld_relaxed_int(&a.err->code);
-        if (!run64<DIR>(a, sR)) break;
+        if (!run64<DIR>(a, sR, prod)) break;
     }
     leave(a.ctl);
 }
@@ -455,6 +527,24 @@ __device__ __forceinline__ void ld_row(const float* p, float (&y)[K]) {
             y[h] = __uint_as_float(a0); y[h + 1] = __uint_as_float(a1);
             y[h + 2] = __uint_as_float(a2); y[h + 3] = __uint_as_float(a3);
         }
+    }
+}
+
+// The same where `on` (elsewhere y stays as it is), by predicate and not by branch.
+template <int K>
+__device__ __forceinline__ void ld_row_if(bool on, const float* p, float (&y)[K]) {
+    const unsigned f = on;
+    if constexpr (K == 1) {
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %1, 0; @q ld.relaxed.gpu.global.b32 %0, [%2];}"
+                     : "+f"(y[0]) : "r"(f), "l"(p) : "memory");
+    } else if constexpr (K == 2) {
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.relaxed.gpu.global.v2.b32 {%0,%1}, [%3];}"
+                     : "+f"(y[0]), "+f"(y[1]) : "r"(f), "l"(p) : "memory");
+    } else {
+#pragma unroll
+        for (int h = 0; h < K; h += 4)
+            asm volatile("{.reg .pred q; setp.ne.u32 q, %4, 0; @q ld.relaxed.gpu.global.v4.b32 {%0,%1,%2,%3}, [%5];}"
+                         : "+f"(y[h]), "+f"(y[h + 1]), "+f"(y[h + 2]), "+f"(y[h + 3]) : "r"(f), "l"(p + h) : "memory");
     }
 }
 
@@ -494,6 +584,12 @@ struct stage_data32 {
     float ww[batch_of<K>::value];
 };
 
+// Entry t of a row in processing order: plan order forward; backward the plan
+// lists the newest dependency first, so it is walked from its end.
+__device__ __forceinline__ uint32_t entry_at(const lane_view& v, uint32_t t, bool back) {
+    return v.q + (back ? v.len - 1u - t : t);
+}
+
 // Weight of plan entry e: fp32, or the binary16 value widened (exact).
 template <bool H>
 __device__ __forceinline__ float weight32(const sweep_args<float>& a, uint32_t e) {
@@ -501,7 +597,7 @@ __device__ __forceinline__ float weight32(const sweep_args<float>& a, uint32_t e
     else return __ldg(a.val + e);
 }
 
-template <int K, bool H>
+template <int DIR, int K, bool H>
 __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const double* in64, const stage_desc& ds,
                                             stage_data32<K>& s) {
     constexpr int B = batch_of<K>::value;
@@ -514,7 +610,11 @@ __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const do
 #pragma unroll
     for (int k = 0; k < B; ++k) {
         const uint32_t t = (static_cast<uint32_t>(k) << v.lg) + v.u;
-        if (t < v.len) { s.jj[k] = __ldg(a.idx + v.q + t); s.ww[k] = weight32<H>(a, v.q + t); }
+        if (t < v.len) {
+            const uint32_t e = entry_at(v, t, DIR == 1);
+            s.jj[k] = __ldg(a.idx + e);
+            s.ww[k] = weight32<H>(a, e);
+        }
     }
     if (v.valid && v.u == 0) {
         const size_t base = static_cast<size_t>(v.row) * K;
@@ -537,6 +637,52 @@ __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const do
     }
 }
 
+// a / d in fp32, correctly rounded, for a divisor known before the dividend: a
+// Newton step on a r, r = RN(1 / d), makes the quotient faithful, and a faithful
+// quotient corrected by its exact remainder times r is the rounded one
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990). Divisors and dividends whose reciprocal, quotient or
+// remainder leaves the normal range divide.
+struct recip32 {
+    float d, r;
+    unsigned span;   // exponents of a that take the short way: [67, 67 + span)
+    __device__ __forceinline__ float quotient(float a) const {
+        float q = __fmul_rn(a, r);
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
+        if (((__float_as_uint(a) >> 23) & 0xffu) - 67u >= span) q = __fdiv_rn(a, d);
+        return q;
+    }
+};
+__device__ __forceinline__ recip32 recip_of(float d) {
+    return {d, __frcp_rn(d), ((__float_as_uint(d) >> 23) & 0xffu) - (127u - 40u) < 80u ? 120u : 0u};
+}
+
+// Sums nk operand rows into acc in order once the warp has all of them (oldest
+// dependency first): ld(on, j, y) loads operand row j into y where on. Straight
+// line code with one vote a pass, since a pass over the pending rows is what
+// stands between the last operand's arrival and the row. Narrow rows wait on
+// the newest pending one (see kLight). Returns false when the warp must drain.
+template <int B, int K, class Ld, class Idle>
+__device__ __forceinline__ bool gather32(uint32_t nk, const uint32_t (&jj)[B], const float (&ww)[B], float (&yv)[B][K],
+                                         float (&acc)[K], Ld&& ld, Idle&& idle) {
+    for (;;) {
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < B; ++k) open |= static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
+        if (!__any_sync(kFull, open)) break;
+        if (idle()) return false;
+#pragma unroll
+        for (int k = 0; k < B; ++k) ld(static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]), jj[k], yv[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+        if (static_cast<uint32_t>(k) < nk)
+#pragma unroll
+            for (int r = 0; r < K; ++r) acc[r] = __fmaf_rn(ww[k], yv[k][r], acc[r]);
+    return true;
+}
+
 template <int DIR, int K, bool H>
 __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K>& s) {
     constexpr int B = batch_of<K>::value;
@@ -547,42 +693,33 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
     float acc[K];
 #pragma unroll
     for (int r = 0; r < K; ++r) acc[r] = 0.0f;
+    const recip32 inv = recip_of(s.d);
     idle_clock clk;
     for (uint32_t jb = 0; jb < Jmax; jb += B) {
         if (jb > 0) {
 #pragma unroll
             for (int k = 0; k < B; ++k) {
                 const uint32_t t = ((jb + k) << v.lg) + v.u;
-                if (t < v.len) { s.jj[k] = __ldg(a.idx + v.q + t); s.ww[k] = weight32<H>(a, v.q + t); }
+                if (t < v.len) {
+                    const uint32_t e = entry_at(v, t, DIR == 1);
+                    s.jj[k] = __ldg(a.idx + e);
+                    s.ww[k] = weight32<H>(a, e);
+                }
             }
         }
         // this lane's entries in the batch: steps 0 .. nk-1
         const uint32_t t0 = (jb << v.lg) + v.u;
         const uint32_t nk = t0 < v.len ? min(static_cast<uint32_t>(B), ((v.len - t0 - 1u) >> v.lg) + 1u) : 0u;
         float yv[B][K];
+        const auto ld = [&](bool on, uint32_t j, float (&y)[K]) { ld_row_if<K>(on, a.out + static_cast<size_t>(j) * K, y); };
 #pragma unroll
-        for (int k = 0; k < B; ++k)
-            if (static_cast<uint32_t>(k) < nk) ld_row<K>(a.out + static_cast<size_t>(s.jj[k]) * K, yv[k]);
-        // each lane consumes its own entries in order as they arrive
-        uint32_t kpos = 0;
-        for (;;) {
-            const uint32_t before = kpos;
+        for (int k = 0; k < B; ++k) {
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                if (kpos == static_cast<uint32_t>(k) && kpos < nk && row_ready<K>(yv[k])) {
-#pragma unroll
-                    for (int r = 0; r < K; ++r) acc[r] = __fmaf_rn(s.ww[k], yv[k][r], acc[r]);
-                    ++kpos;
-                }
-            }
-            if (__all_sync(kFull, kpos >= nk)) break;
-            if (__any_sync(kFull, kpos != before)) clk.spins = 0;
-            else if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
-#pragma unroll
-            for (int k = 0; k < B; ++k)
-                if (static_cast<uint32_t>(k) >= kpos && static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]))
-                    ld_row<K>(a.out + static_cast<size_t>(s.jj[k]) * K, yv[k]);
+            for (int r = 0; r < K; ++r) yv[k][r] = 0.0f;
+            ld(static_cast<uint32_t>(k) < nk, s.jj[k], yv[k]);
         }
+        if (!gather32<B, K>(nk, s.jj, s.ww, yv, acc, ld, [&] { return clk.idle(a.err, a.budget_ns, where, v.row); })) return false;
+        clk.spins = 0;
     }
     // fixed butterfly over the group's lanes
     for (unsigned o = v.G >> 1; o > 0; o >>= 1)
@@ -591,12 +728,8 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
     if (v.valid && v.u == 0) {
         float y[K];
 #pragma unroll
-        for (int r = 0; r < K; ++r) y[r] = __fdiv_rn(s.rhs[r] - acc[r], s.d);
+        for (int r = 0; r < K; ++r) y[r] = inv.quotient(s.rhs[r] - acc[r]);
         st_row<K>(a.out + static_cast<size_t>(v.row) * K, y);
-        if (a.copy_out) {
-#pragma unroll
-            for (int r = 0; r < K; ++r) a.copy_out[static_cast<size_t>(v.row) * K + r] = y[r];
-        }
         if (a.reset) {   // re-arm after the right-hand side was consumed (see run64)
             float sent[K];
 #pragma unroll
@@ -616,12 +749,12 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_df32(const sweep_args<floa
     stage_desc dD;
     load_desc(a, cc.next(a), dD);
     stage_data32<K> sL;
-    load_data32<K, H>(a, in64, dD, sL);
+    load_data32<DIR, K, H>(a, in64, dD, sL);
     load_desc(a, cc.next(a), dD);
     int bad = 0;   // the error word, read one item late
     while (sL.v.c < a.n_items) {
         stage_data32<K> sR = sL;
-        load_data32<K, H>(a, in64, dD, sL);
+        load_data32<DIR, K, H>(a, in64, dD, sL);
         load_desc(a, cc.next(a), dD);
         if (__shfl_sync(kFull, bad, 0)) break;
         if (lane == 0) bad = ld_relaxed_int(&a.err->code);
@@ -804,162 +937,545 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_dw32(const sweep_args<floa
 }
 
 // ---------------------------------------------------------------------------
-// Serial segment: one block solves the run of small trailing levels (forward:
-// after the dataflow launch; backward: before it) level by level, values in
-// shared memory, __syncthreads between levels. Each warp solves its rows (the
-// segment rows round-robin over the warps, in processing order) with all 32
-// lanes, and prefetches its next row while working on the current one.
+// Cluster tail: the run of narrow levels at the end of the elimination
+// (forward: after the dataflow launch; backward: before it), one thread-block
+// cluster per column slice (KC columns). Every CTA of the cluster
+// holds a copy of the tail's solution in shared memory; the warp that solves a
+// row stores it into all the copies (distributed shared memory) and into the
+// output vector, and a row waits by polling its own SM's copy.
+// What bounds it: the chain of levels. In the dataflow kernels a narrow level
+// costs a store, an L2 round trip and the polls of every warp that waits
+// further down (0.7 us alone, 1.1 us and more with the whole grid polling);
+// here a hop is a DSM store and a shared-memory poll, and no other SM sees it.
+// What is left of a hop (0.45 us in fp32) is the instructions between the
+// operand's arrival and the store, so those paths are short: a row's lanes all
+// hold its sum, right-hand side and divisor, the batches of a row are compiled
+// for 1, 2, 4 and 8 steps, the divisor's reciprocal, the store addresses and
+// everything else that does not depend on the operands are ready before.
+// Measured, one sweep pair (us), all levels in the dataflow launch before ->
+// with the tail: fp64 6-regular n = 100003 2849 -> 1230, 61^3 grid 653 -> 346,
+// 128^3 grid 1524 -> 870, 256^2 grid 180 -> 117; fp32 6-regular 2131 -> 571,
+// 61^3 412 -> 214, 128^3 1019 -> 622; k = 16 6-regular 4866 -> 905.
+// Items go to the cluster's warps round robin in level order (no claims), so
+// the lowest unfinished item is always its warp's next one and, all CTAs of a
+// cluster being resident together, progress never depends on scheduling. A warp
+// has the operands from outside the tail, entries, right-hand sides and
+// descriptors of its next items in flight while it waits for the current one.
 
-constexpr int kSegThreads = 512;
-constexpr uint64_t kBox = 0xFFF6000000000000ull;   // NaN box carrying a segment-local index
+constexpr int kTailThreads = 256;
 
-__device__ __forceinline__ double box_index(uint32_t i) { return __longlong_as_double(static_cast<long long>(kBox | i)); }
-__device__ __forceinline__ bool is_box(double v) {
-    return (static_cast<unsigned long long>(__double_as_longlong(v)) & 0xFFFF000000000000ull) == kBox;
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
 }
-__device__ __forceinline__ uint32_t unbox(double v) {
-    return static_cast<uint32_t>(static_cast<unsigned long long>(__double_as_longlong(v)) & 0xffffffffull);
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_addr(unsigned local, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void near_ld_if(bool on, unsigned p, double& y) {
+    unsigned long long v = static_cast<unsigned long long>(__double_as_longlong(y));
+    asm volatile("{.reg .pred q; setp.ne.u32 q, %1, 0; @q ld.relaxed.cluster.shared::cta.b64 %0, [%2];}"
+                 : "+l"(v) : "r"(static_cast<unsigned>(on)), "r"(p) : "memory");
+    y = __longlong_as_double(static_cast<long long>(v));
+}
+__device__ __forceinline__ void peer_st(unsigned p, double y) {
+    asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(p), "l"(__double_as_longlong(y)) : "memory");
+}
+template <int KC>
+__device__ __forceinline__ void near_ld_row_if(bool on, unsigned p, float (&y)[KC]) {
+    const unsigned f = on;
+    if constexpr (KC == 1)
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %1, 0; @q ld.relaxed.cluster.shared::cta.b32 %0, [%2];}"
+                     : "+f"(y[0]) : "r"(f), "r"(p) : "memory");
+    else if constexpr (KC == 2)
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.relaxed.cluster.shared::cta.v2.b32 {%0,%1}, [%3];}"
+                     : "+f"(y[0]), "+f"(y[1]) : "r"(f), "r"(p) : "memory");
+    else
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %4, 0; @q ld.relaxed.cluster.shared::cta.v4.b32 {%0,%1,%2,%3}, [%5];}"
+                     : "+f"(y[0]), "+f"(y[1]), "+f"(y[2]), "+f"(y[3]) : "r"(f), "r"(p) : "memory");
+}
+template <int KC>
+__device__ __forceinline__ void peer_st_row(unsigned p, const float (&y)[KC]) {
+    if constexpr (KC == 1)
+        asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(p), "r"(__float_as_uint(y[0])) : "memory");
+    else if constexpr (KC == 2)
+        asm volatile("st.relaxed.cluster.shared::cluster.v2.b32 [%0], {%1,%2};"
+                     ::"r"(p), "r"(__float_as_uint(y[0])), "r"(__float_as_uint(y[1])) : "memory");
+    else
+        asm volatile("st.relaxed.cluster.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};"
+                     ::"r"(p), "r"(__float_as_uint(y[0])), "r"(__float_as_uint(y[1])), "r"(__float_as_uint(y[2])),
+                       "r"(__float_as_uint(y[3])) : "memory");
 }
 
-struct seg_slot {
-    uint32_t i, r, q, len;
-    double rhs, d;
-    double pv[kBatch];   // product (operand outside the segment, final) or the boxed segment index
+// Polls of shared memory disturb no other SM and the loop around them has to be
+// short: the error word and the time budget are looked at every 4096th poll.
+struct near_clock {
+    unsigned spins = 0;
+    unsigned long long t0 = 0;
+    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row) {
+        if ((++spins & 4095u) != 0) return false;
+        if (t0 == 0) t0 = globaltimer();
+        return wait_must_stop(err, __shfl_sync(kFull, t0, 0), budget, where, row);
+    }
+};
+
+__device__ __forceinline__ double quiet_nan(double) { return __longlong_as_double(0x7ff8000000000000ll); }
+__device__ __forceinline__ float quiet_nan(float) { return __uint_as_float(0x7fc00000u); }
+
+// The cluster's column slice and the warp's place among the cluster's warps.
+struct tail_seat {
+    unsigned col0, warp, warps, base;   // base: shared address of the CTA's copy
+};
+
+__device__ __forceinline__ tail_seat take_seat(int kc, unsigned base) {
+    const unsigned cs = cluster_size();
+    tail_seat t;
+    t.col0 = (blockIdx.x / cs) * kc;
+    t.warp = (threadIdx.x >> 5) * cs + cluster_rank();   // consecutive items on different SMs
+    t.warps = cs * (kTailThreads / 32);
+    t.base = base;
+    return t;
+}
+
+// Descriptor of item c of the tail (nothing for c >= item1).
+template <class T>
+__device__ __forceinline__ void tail_desc(const tail_args<T>& p, uint32_t c, stage_desc& d) {
+    const unsigned lane = threadIdx.x & 31u;
+    d.c = c;
+    d.info = 0; d.row = kNoRowDev; d.q = 0; d.e = 0;
+    if (c < p.item1) {
+        const size_t pos = static_cast<size_t>(c) * 32 + lane;
+        d.info = __ldg(p.info + c);
+        d.row = __ldg(p.ord + pos);
+        d.q = __ldg(p.ptr + pos);
+        d.e = __ldg(p.ptr + pos + 1);
+    }
+}
+
+// Lane view of a tail item: a factor plan's rows take all 32 lanes (its lane
+// groups are sized for throughput; here few rows mean few entries per lane).
+__device__ __forceinline__ lane_view spread_view(stage_desc d) {
+    const unsigned rows = d.info & 0xffu;
+    if (rows) {
+        const unsigned lg = 5u - (32u - __clz(rows - 1u));   // 32 >> lg >= rows
+        d.info = (d.info & ~0xff00u) | (lg << 8);
+    }
+    return view_of(d);
+}
+
+// Stores a solved row's value into every copy: lane u of the row's group into
+// copies u, u + G, ...; at: the row's shared address, to: its address in copy u.
+template <class St>
+__device__ __forceinline__ void push_row(const lane_view& v, unsigned cs, unsigned at, unsigned to, St&& st) {
+    if (v.valid && v.u < cs) st(to);
+    for (unsigned q = v.u + v.G; q < cs; q += v.G)
+        if (v.valid) st(peer_addr(at, q));
+}
+
+// ---- fp64: the reference's sum order, as run64
+
+struct near_row64 {
+    lane_view v;
+    double rhs, d;               // every lane of the group
+    uint32_t jj[kBatch];
     float ww[kBatch];
 };
 
-__device__ __forceinline__ void seg_batch64(const sweep_args<double>& a, const seg_slot& s, uint32_t jb,
-                                            double (&pv)[kBatch], float (&ww)[kBatch]) {
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t s0 = a.seg_first, s1 = a.seg_first + a.seg_rows;
+__device__ __forceinline__ void near_entries64(const tail_args<double>& p, const lane_view& v, uint32_t jb, near_row64& s) {
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
-        const uint32_t t = ((jb + k) << 5) + lane;
-        pv[k] = 0.0;
-        ww[k] = 0.0f;
-        if (t < s.len) {
-            const uint32_t j = __ldg(a.seg_idx + s.q + t);
-            const float w = __ldg(a.seg_val + s.q + t);
-            ww[k] = w;
-            pv[k] = (j >= s0 && j < s1) ? box_index(j - s0) : __dmul_rn(static_cast<double>(w), a.out[j]);
+        const uint32_t t = ((jb + k) << v.lg) + v.u;
+        s.jj[k] = 0xffffffffu;
+        s.ww[k] = 0.0f;
+        if (t < v.len) { s.jj[k] = __ldg(p.idx + v.q + t); s.ww[k] = __ldg(p.val + v.q + t); }
+    }
+}
+
+__device__ __forceinline__ void near_data64(const tail_args<double>& a, const stage_desc& ds, near_row64& s) {
+    // rows of one lane each in the plan keep it when there are more than eight (the 4-way sum needs 4 lanes a row)
+    s.v = (ds.info & 0xff00u) == 0 && (ds.info & 0xffu) > 8u ? view_of(ds) : spread_view(ds);
+    s.rhs = 0.0; s.d = 1.0;
+    near_entries64(a, s.v, 0, s);
+    if (s.v.valid) {
+        s.rhs = a.in[s.v.row];
+        s.d = static_cast<double>(__ldg(a.val + s.v.q + s.v.len));
+    }
+}
+
+// Operands of a batch from outside the tail (complete before the launch); the
+// tail's own are marked as to come.
+__device__ __forceinline__ void near_outside64(const tail_args<double>& a, const near_row64& s, double (&y)[kBatch]) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+        y[k] = s.jj[k] == 0xffffffffu ? 0.0 : sent_of(0.0);
+        if (s.jj[k] < a.first) {
+            y[k] = a.out[s.jj[k]];
+            if (is_sent(y[k])) y[k] = quiet_nan(0.0);   // the launch before this one failed
         }
     }
 }
 
-__device__ __forceinline__ void seg_fetch64(const sweep_args<double>& a, uint32_t i, seg_slot& s) {
-    s.i = i;
-    s.len = 0;
-    if (i >= a.seg_rows) return;
-    s.r = __ldg(a.seg_row + i);
-    s.q = __ldg(a.seg_ptr + i);
-    s.len = __ldg(a.seg_ptr + i + 1) - s.q - 1u;
-    seg_batch64(a, s, 0, s.pv, s.ww);
-    if ((threadIdx.x & 31u) == 0) {
-        s.rhs = a.in[s.r];
-        s.d = static_cast<double>(__ldg(a.seg_val + s.q + s.len));
-    }
-}
-
-__device__ __forceinline__ void seg_solve64(const sweep_args<double>& a, seg_slot& s, bool thin, double* segv) {
+// One batch of NB steps (NB >= the warp's steps in it) of group rows: products
+// into shared memory as the operands arrive; while some are missing the leading
+// ones are consumed, and the rest when the last is in. Every lane runs the
+// chain u mod 4 of its row (thin) or the serial sum (fat): the same values, no
+// divergence.
+template <int NB>
+__device__ __forceinline__ bool near_batch64(const tail_args<double>& a, const tail_seat& t, const near_row64& s,
+                                             double (&y)[kBatch], uint32_t jb, uint32_t gend, int where, double* prod,
+                                             uint32_t& at, double& sum, near_clock& clk) {
+    const lane_view& v = s.v;
     const unsigned lane = threadIdx.x & 31u;
-    const uint32_t J = (s.len + 31u) >> 5;
-    const uint32_t gend = thin ? (s.len & ~3u) : 0u;
-    exact_state e;
-    for (uint32_t jb = 0; jb < J; jb += kBatch) {
-        if (jb > 0) seg_batch64(a, s, jb, s.pv, s.ww);
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            double p = s.pv[k];
-            if (is_box(p)) p = __dmul_rn(static_cast<double>(s.ww[k]), segv[unbox(p)]);
-            exact_step<5>(thin, jb + k < J, lane, (jb + k) << 5, s.len, gend, p, e);
+    const double* pr = prod + v.G * v.gid;
+    const unsigned W = v.thin ? 4u : 1u, c = v.thin ? (v.u & 3u) : 0u;
+    const auto prod_of = [&](uint32_t e) { return pr[32u * ((e >> v.lg) - jb) + (e & (v.G - 1u))]; };
+    const auto take = [&](uint32_t upto) {
+        while (at + 4u * W <= upto) {
+            const double q0 = prod_of(at + c), q1 = prod_of(at + W + c), q2 = prod_of(at + 2u * W + c), q3 = prod_of(at + 3u * W + c);
+            sum = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(sum, q0), q1), q2), q3);
+            at += 4u * W;
         }
+        while (at + W <= upto) {
+            sum = __dadd_rn(sum, prod_of(at + c));
+            at += W;
+        }
+    };
+    bool w[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) w[k] = true;
+    for (;;) {
+        bool open = false, got = false;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) near_ld_if(w[k] && is_sent(y[k]), t.base + (s.jj[k] - a.first) * 8u, y[k]);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            if (w[k] && !is_sent(y[k])) {
+                prod[32 * k + lane] = __dmul_rn(static_cast<double>(s.ww[k]), y[k]);
+                w[k] = false;
+                got = true;
+            }
+            open |= w[k];
+        }
+        const bool more = __any_sync(kFull, open);
+        if (!more) break;
+        if (__any_sync(kFull, got)) {
+            // the entries before the group's first missing one
+            unsigned pend = 0;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) pend |= w[k] ? 1u << k : 0u;
+            __syncwarp();
+            const uint32_t st = static_cast<uint32_t>(__ffs(__reduce_or_sync(kFull, pend))) - 1u;
+            const unsigned miss = __ballot_sync(kFull, (pend >> st) & 1u) >> (v.gid << v.lg);
+            const unsigned mine = v.lg == 5 ? miss : miss & ((1u << v.G) - 1u);
+            take(min(gend, ((jb + st) << v.lg) + (mine ? static_cast<uint32_t>(__ffs(mine)) - 1u : v.G)));
+            clk = near_clock{};
+        }
+        if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
     }
-    const double s1 = __shfl_sync(kFull, e.s, 1), s2 = __shfl_sync(kFull, e.s, 2), s3 = __shfl_sync(kFull, e.s, 3);
-    const double total = !thin ? e.s : (e.combined ? e.sum : dadd4(e.s, s1, s2, s3));
-    if (lane == 0) {
-        double rhs = s.rhs;
+    __syncwarp();
+    take(min(gend, (jb + NB) << v.lg));
+    return true;
+}
+
+__device__ __forceinline__ bool near_group64(const tail_args<double>& a, const tail_seat& t, near_row64& s,
+                                             double (&y)[kBatch], int where, double* prod, double& total) {
+    const lane_view& v = s.v;
+    const uint32_t Jmax = __reduce_max_sync(kFull, (v.len + v.G - 1u) >> v.lg);
+    const uint32_t gend = v.thin ? (v.len & ~3u) : v.len;   // entries the chains take
+    double sum = 0.0;
+    uint32_t at = 0, jb = 0;
+    near_clock clk;
+    for (; jb + kBatch < Jmax; jb += kBatch) {
+        if (!near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum, clk)) return false;
+        near_entries64(a, v, jb + kBatch, s);
+        near_outside64(a, s, y);
+        __syncwarp();   // the batch's products have been read
+    }
+    const uint32_t nb = Jmax - jb;
+    const bool ok = nb <= 1 ? near_batch64<1>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
+                  : nb <= 2 ? near_batch64<2>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
+                  : nb <= 4 ? near_batch64<4>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
+                            : near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum, clk);
+    if (!ok) return false;
+    if (v.thin) {   // (s0 + s1) + (s2 + s3), then the <= 3 entries left (in the row's last batch)
+        sum = __dadd_rn(sum, __shfl_xor_sync(kFull, sum, 1));
+        sum = __dadd_rn(sum, __shfl_xor_sync(kFull, sum, 2));
+        const double* pr = prod + v.G * v.gid;
+        for (uint32_t e = gend; e < v.len; ++e) sum = __dadd_rn(sum, pr[32u * ((e >> v.lg) - jb) + (e & (v.G - 1u))]);
+    }
+    __syncwarp();   // the products have been read
+    total = sum;
+    return true;
+}
+
+// More than eight rows of <= kBatch entries: a lane each.
+__device__ __forceinline__ bool near_lane64(const tail_args<double>& a, const tail_seat& t, const near_row64& s,
+                                            double (&y)[kBatch], int where, double& total) {
+    const lane_view& v = s.v;
+    near_clock clk;
+    for (;;) {
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) near_ld_if(is_sent(y[k]), t.base + (s.jj[k] - a.first) * 8u, y[k]);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) open |= is_sent(y[k]);
+        if (!__any_sync(kFull, open)) break;
+        if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
+    }
+    double p[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) p[k] = __dmul_rn(static_cast<double>(s.ww[k]), y[k]);
+    total = lane_sum64(p, v.len, __reduce_max_sync(kFull, v.len), v.thin ? (v.len & ~3u) : 0u);
+    return true;
+}
+
+__global__ void __launch_bounds__(kTailThreads, 1) k_tail64(const tail_args<double> a, int where) {
+    if (a.skip && *a.skip) return;
+    extern __shared__ __align__(16) double near_y[];
+    __shared__ __align__(16) double prods[kTailThreads / 32][32 * kBatch];
+    double* prod = prods[threadIdx.x >> 5];
+    const tail_seat t = take_seat(1, static_cast<unsigned>(__cvta_generic_to_shared(near_y)));
+    for (uint32_t i = threadIdx.x; i < a.rows; i += kTailThreads) near_y[i] = sent_of(0.0);
+    cluster_barrier();
+    const unsigned cs = cluster_size();
+    uint32_t c = a.item0 + t.warp;
+    stage_desc ds;
+    near_row64 s0, s1;
+    double y0[kBatch], y1[kBatch];
+    tail_desc(a, c, ds);
+    near_data64(a, ds, s0);
+    tail_desc(a, c + t.warps, ds);
+    near_data64(a, ds, s1);
+    tail_desc(a, c + 2 * t.warps, ds);
+    near_outside64(a, s0, y0);
+    while (s0.v.c < a.item1) {
+        near_outside64(a, s1, y1);   // the next item's indices came in with the last one
+        const lane_view& v = s0.v;
+        const recip64 inv = recip_of(s0.d);
+        const unsigned at = t.base + (v.valid ? v.row - a.first : 0u) * 8u, to = peer_addr(at, v.u & (cs - 1u));
+        double rhs = s0.rhs, total = 0.0;
         if (a.rhs_sub) rhs = __dsub_rn(rhs, *a.rhs_sub);
-        const double y = __ddiv_rn(__dsub_rn(rhs, total), s.d);
-        segv[s.r - a.seg_first] = y;
-        a.out[s.r] = y;
-        if (a.copy_out) a.copy_out[s.r] = y;
-        if (a.reset) a.reset[s.r] = sent_of(0.0);
+        if (!(v.lg == 0 ? near_lane64(a, t, s0, y0, where, total) : near_group64(a, t, s0, y0, where, prod, total))) break;
+        const double y = inv.quotient(__dsub_rn(rhs, total));
+        push_row(v, cs, at, to, [&](unsigned p) { peer_st(p, y); });
+        if (v.valid && v.u == 0) {
+            a.out[v.row] = y;
+            if (a.copy_out) a.copy_out[v.row] = y;
+            if (a.reset) a.reset[v.row] = sent_of(0.0);
+        }
+        s0 = s1;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) y0[k] = y1[k];
+        near_data64(a, ds, s1);
+        c += t.warps;
+        tail_desc(a, c + 2 * t.warps, ds);
+    }
+    cluster_barrier();   // no CTA leaves while another may still store into its copy
+}
+
+// ---- fp32: KC columns of the k per cluster, every lane adding its entries in
+// order (oldest dependency first), the lanes' sums by a fixed butterfly
+
+template <int KC>
+struct near_row32 {
+    lane_view v;
+    float rhs[KC], d;            // every lane of the group
+    uint32_t jj[kBatch];
+    float ww[kBatch];
+};
+
+template <bool H>
+__device__ __forceinline__ float tail_weight(const tail_args<float>& p, uint32_t e) {
+    if constexpr (H) return __half2float(__ushort_as_half(__ldg(p.val16 + e)));
+    else return __ldg(p.val + e);
+}
+
+template <int KC, bool H>
+__device__ __forceinline__ void near_entries32(const tail_args<float>& p, const lane_view& v, uint32_t jb, bool back,
+                                               near_row32<KC>& s) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+        const uint32_t t = ((jb + k) << v.lg) + v.u;
+        s.jj[k] = 0xffffffffu;
+        s.ww[k] = 0.0f;
+        if (t < v.len) {
+            const uint32_t e = entry_at(v, t, back);
+            s.jj[k] = __ldg(p.idx + e);
+            s.ww[k] = tail_weight<H>(p, e);
+        }
     }
 }
 
-__global__ void __launch_bounds__(kSegThreads, 1) k_seg64(const sweep_args<double> a) {
-    if (a.skip && *a.skip) return;
-    if (a.err->code != 0) return;
-    extern __shared__ double segv[];
-    const unsigned warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    seg_slot cur, nxt;
-    seg_fetch64(a, warp, cur);
-    for (uint32_t l = 0; l < a.seg_levels; ++l) {
-        const uint32_t w0 = __ldg(a.seg_lvl + l), hi = __ldg(a.seg_lvl + l + 1) & 0x7fffffffu;
-        const bool thin = (w0 >> 31) != 0;
-        while (cur.i < hi) {
-            seg_fetch64(a, cur.i + nw, nxt);
-            seg_solve64(a, cur, thin, segv);
-            cur = nxt;
+template <int KC, bool H>
+__device__ __forceinline__ void near_data32(const tail_args<float>& a, const tail_seat& t, const stage_desc& ds, bool back,
+                                            near_row32<KC>& s) {
+    if (a.wide) {   // a batch plan's row keeps its entry lanes, and with them the dataflow launch's sums
+        s.v = view_of(ds);   // (k <= 4: one column lane)
+    } else {
+        s.v = spread_view(ds);
+    }
+    const lane_view& v = s.v;
+    s.d = 1.0f;
+#pragma unroll
+    for (int r = 0; r < KC; ++r) s.rhs[r] = 0.0f;
+    near_entries32<KC, H>(a, v, 0, back && !a.wide, s);   // batch plans list the oldest dependency first both ways
+    if (v.valid) {
+        const size_t base = static_cast<size_t>(v.row) * a.k + t.col0;
+        if (a.in64) {
+#pragma unroll
+            for (int r = 0; r < KC; ++r) {
+                double x = a.in64[base + r];
+                if (a.rhs_sub) x -= a.rhs_sub[t.col0 + r];
+                s.rhs[r] = static_cast<float>(x);
+            }
+        } else if (H && back) {   // fp16 storage: the backward input times inv_scale^2, in fp64, rounded once
+            const double sc = a.scale2[v.row];
+#pragma unroll
+            for (int r = 0; r < KC; ++r) s.rhs[r] = static_cast<float>(static_cast<double>(a.in[base + r]) * sc);
+        } else {
+#pragma unroll
+            for (int r = 0; r < KC; ++r) s.rhs[r] = a.in[base + r];
         }
-        __syncthreads();
+        s.d = H ? __ldg(a.diag16 + v.row) : __ldg(a.val + v.q + v.len);
     }
 }
 
-// fp32, K right-hand sides: lanes stride the row's entries, operands from
-// shared memory (inside the segment) or the output vector (final), fixed
-// butterfly.
-template <int K>
-__global__ void __launch_bounds__(kSegThreads, 1) k_seg32(const sweep_args<float> a, const double* in64) {
+// Operand rows of a batch from outside the tail (complete before the launch);
+// the tail's own are marked as to come, absent ones are 0 (with weight 0).
+template <int KC>
+__device__ __forceinline__ void near_outside32(const tail_args<float>& a, const tail_seat& t, const near_row32<KC>& s,
+                                               float (&yv)[kBatch][KC]) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+        const uint32_t j = s.jj[k];
+#pragma unroll
+        for (int r = 0; r < KC; ++r) yv[k][r] = j == 0xffffffffu ? 0.0f : sent_of(0.0f);
+        if (j >= a.first) continue;
+        const float* src = a.out + static_cast<size_t>(j) * a.k + t.col0;
+        if constexpr (KC == 4) {
+            const float4 q = *reinterpret_cast<const float4*>(src);
+            yv[k][0] = q.x; yv[k][1] = q.y; yv[k][2] = q.z; yv[k][3] = q.w;
+        } else if constexpr (KC == 2) {
+            const float2 q = *reinterpret_cast<const float2*>(src);
+            yv[k][0] = q.x; yv[k][1] = q.y;
+        } else {
+            yv[k][0] = src[0];
+        }
+#pragma unroll
+        for (int r = 0; r < KC; ++r)
+            if (is_sent(yv[k][r])) yv[k][r] = quiet_nan(0.0f);   // the launch before this one failed
+    }
+}
+
+// One batch of NB steps (NB >= the warp's steps in it): polls until every
+// operand is in, then the sums in straight line.
+template <int KC, int NB>
+__device__ __forceinline__ bool near_batch32(const tail_args<float>& a, const tail_seat& t, const near_row32<KC>& s,
+                                             float (&yv)[kBatch][KC], int where, float (&acc)[KC], near_clock& clk) {
+    for (;;) {
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            near_ld_row_if<KC>(!row_ready<KC>(yv[k]), t.base + (s.jj[k] - a.first) * (4u * KC), yv[k]);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) open |= !row_ready<KC>(yv[k]);
+        if (!__any_sync(kFull, open)) break;
+        if (clk.idle(a.err, a.budget_ns, where, s.v.row)) return false;
+    }
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+#pragma unroll
+        for (int r = 0; r < KC; ++r) acc[r] = __fmaf_rn(s.ww[k], yv[k][r], acc[r]);
+    return true;
+}
+
+template <int KC, bool H>
+__device__ __forceinline__ bool near_run32(const tail_args<float>& a, const tail_seat& t, near_row32<KC>& s, bool back,
+                                           int where, float (&yv)[kBatch][KC], float (&acc)[KC]) {
+    const lane_view& v = s.v;
+    const uint32_t Jmax = __reduce_max_sync(kFull, (v.len + v.G - 1u) >> v.lg);
+#pragma unroll
+    for (int r = 0; r < KC; ++r) acc[r] = 0.0f;
+    near_clock clk;
+    uint32_t jb = 0;
+    for (; jb + kBatch < Jmax; jb += kBatch) {
+        if (!near_batch32<KC, kBatch>(a, t, s, yv, where, acc, clk)) return false;
+        near_entries32<KC, H>(a, v, jb + kBatch, back && !a.wide, s);
+        near_outside32<KC>(a, t, s, yv);
+    }
+    const uint32_t nb = Jmax - jb;
+    const bool ok = nb <= 1 ? near_batch32<KC, 1>(a, t, s, yv, where, acc, clk)
+                  : nb <= 2 ? near_batch32<KC, 2>(a, t, s, yv, where, acc, clk)
+                  : nb <= 4 ? near_batch32<KC, 4>(a, t, s, yv, where, acc, clk)
+                            : near_batch32<KC, kBatch>(a, t, s, yv, where, acc, clk);
+    if (!ok) return false;
+#pragma unroll
+    for (unsigned i = 5; i-- > 0;)
+        if (v.lg > i)
+#pragma unroll
+            for (int r = 0; r < KC; ++r) acc[r] += __shfl_xor_sync(kFull, acc[r], 1 << i);
+    return true;
+}
+
+template <int KC, bool H>
+__global__ void __launch_bounds__(kTailThreads, 1) k_tail32(const tail_args<float> a, int back) {
     if (a.skip && *a.skip) return;
-    if (a.err->code != 0) return;
-    extern __shared__ float segf[];
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint32_t s0 = a.seg_first, s1 = a.seg_first + a.seg_rows;
-    uint32_t i = warp;
-    for (uint32_t l = 0; l < a.seg_levels; ++l) {
-        const uint32_t hi = __ldg(a.seg_lvl + l + 1) & 0x7fffffffu;
-        for (; i < hi; i += nw) {
-            const uint32_t r = __ldg(a.seg_row + i), q = __ldg(a.seg_ptr + i);
-            const uint32_t len = __ldg(a.seg_ptr + i + 1) - q - 1u;
-            float acc[K];
+    extern __shared__ __align__(16) float near_f[];
+    const tail_seat t = take_seat(KC, static_cast<unsigned>(__cvta_generic_to_shared(near_f)));
+    for (uint32_t i = threadIdx.x; i < a.rows * KC; i += kTailThreads) near_f[i] = sent_of(0.0f);
+    cluster_barrier();
+    const unsigned cs = cluster_size();
+    const int where = back ? kBckSweep32 : kFwdSweep32;
+    uint32_t c = a.item0 + t.warp;
+    stage_desc ds;
+    near_row32<KC> s0, s1;
+    float y0[kBatch][KC], y1[kBatch][KC];
+    tail_desc(a, c, ds);
+    near_data32<KC, H>(a, t, ds, back, s0);
+    tail_desc(a, c + t.warps, ds);
+    near_data32<KC, H>(a, t, ds, back, s1);
+    tail_desc(a, c + 2 * t.warps, ds);
+    near_outside32<KC>(a, t, s0, y0);
+    while (s0.v.c < a.item1) {
+        near_outside32<KC>(a, t, s1, y1);   // the next item's indices came in with the last one
+        const lane_view& v = s0.v;
+        const recip32 inv = recip_of(s0.d);
+        const unsigned at = t.base + (v.valid ? v.row - a.first : 0u) * (4u * KC), to = peer_addr(at, v.u & (cs - 1u));
+        float acc[KC], y[KC];
+        if (!near_run32<KC, H>(a, t, s0, back, where, y0, acc)) break;
 #pragma unroll
-            for (int c = 0; c < K; ++c) acc[c] = 0.0f;
-            for (uint32_t t = lane; t < len; t += 32u) {
-                const uint32_t j = __ldg(a.seg_idx + q + t);
-                const float w = __ldg(a.seg_val + q + t);
-                const float* src = (j >= s0 && j < s1) ? segf + static_cast<size_t>(j - s0) * K
-                                                       : a.out + static_cast<size_t>(j) * K;
+        for (int r = 0; r < KC; ++r) y[r] = inv.quotient(s0.rhs[r] - acc[r]);
+        push_row(v, cs, at, to, [&](unsigned p) { peer_st_row<KC>(p, y); });
+        if (v.valid && v.u == 0) {
+            const size_t base = static_cast<size_t>(v.row) * a.k + t.col0;
+            st_row<KC>(a.out + base, y);
+            if (a.reset) {
+                float sent[KC];
 #pragma unroll
-                for (int c = 0; c < K; ++c) acc[c] = __fmaf_rn(w, src[c], acc[c]);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int c = 0; c < K; ++c) acc[c] += __shfl_xor_sync(kFull, acc[c], o);
-            if (lane == 0) {
-                const size_t base = static_cast<size_t>(r) * K;
-                const float d = __ldg(a.seg_val + q + len);
-#pragma unroll
-                for (int c = 0; c < K; ++c) {
-                    float rhs;
-                    if (in64) {
-                        double x = in64[base + c];
-                        if (a.rhs_sub) x -= a.rhs_sub[c];
-                        rhs = static_cast<float>(x);
-                    } else {
-                        rhs = a.in[base + c];
-                    }
-                    const float y = __fdiv_rn(rhs - acc[c], d);
-                    segf[static_cast<size_t>(r - s0) * K + c] = y;
-                    a.out[base + c] = y;
-                    if (a.copy_out) a.copy_out[base + c] = y;
-                    if (a.reset) a.reset[base + c] = sent_of(0.0f);
-                }
+                for (int r = 0; r < KC; ++r) sent[r] = sent_of(0.0f);
+                st_row<KC>(a.reset + base, sent);
             }
         }
-        __syncthreads();
+        s0 = s1;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+            for (int r = 0; r < KC; ++r) y0[k][r] = y1[k][r];
+        near_data32<KC, H>(a, t, ds, back, s1);
+        c += t.warps;
+        tail_desc(a, c + 2 * t.warps, ds);
     }
+    cluster_barrier();   // no CTA leaves while another may still store into its copy
 }
 
 __global__ void k_fill64(double* p, size_t n, double v) {
@@ -986,23 +1502,108 @@ int occ32() {
     return b0 < b1 ? b0 : b1;
 }
 
+// One cluster per column slice (kc columns).
+template <class F, class A>
+void tail_launch(F* kernel, const tail_args<A>& a, int kc, int cluster, int flag, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(a.k / kc) * static_cast<unsigned>(cluster));
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(a.rows) * kc * sizeof(A);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, a, flag);
+}
+
+template <int KC>
+void tail32_kc(int dir, const tail_args<float>& a, bool fp16, int cluster, cudaStream_t s) {
+    if (fp16) tail_launch(k_tail32<KC, true>, a, KC, cluster, dir, s);
+    else tail_launch(k_tail32<KC, false>, a, KC, cluster, dir, s);
+}
+
+// The tail launch's arguments of a sweep (w.tail set).
+template <class T>
+tail_args<T> tail_args_of(const sweep_args<T>& w) {
+    tail_args<T> a{};
+    a.info = w.info; a.ord = w.ord; a.ptr = w.ptr; a.idx = w.idx; a.val = w.val;
+    a.val16 = w.val16; a.diag16 = w.diag16; a.scale2 = w.in_scale2;
+    a.item0 = w.tail->item0; a.item1 = w.tail->item1; a.first = w.tail->first; a.rows = w.tail->rows;
+    a.in = w.in; a.rhs_sub = w.rhs_sub; a.out = w.out; a.reset = w.reset; a.copy_out = w.copy_out;
+    a.err = w.err; a.skip = w.skip; a.budget_ns = w.budget_ns;
+    return a;
+}
+
+void tail64(int dir, const sweep_args<double>& w, cudaStream_t s) {
+    tail_args<double> a = tail_args_of(w);
+    a.k = 1;
+    tail_launch(k_tail64, a, 1, w.tail->cluster, dir == 0 ? kFwdSweep : kBckSweep, s);
+}
+
+// wide: the plan is a batch plan.
+void tail32(int dir, const sweep_args<float>& w, const double* in64, bool wide, cudaStream_t s) {
+    tail_args<float> a = tail_args_of(w);
+    a.k = w.k; a.in64 = in64;
+    a.wide = wide;
+    const bool fp16 = w.val16 != nullptr;
+    // Up to four clusters: a row's sums and its store are on the chain of levels, so fewer columns a
+    // cluster are faster (batch of k = 4, 6-regular n = 100003, forward / backward: 394 / 414 us with
+    // one cluster of 4 columns, 294 / 299 with four).
+    if (w.k >= 16) tail32_kc<4>(dir, a, fp16, w.tail->cluster, s);
+    else if (w.k == 8) tail32_kc<2>(dir, a, fp16, w.tail->cluster, s);
+    else tail32_kc<1>(dir, a, fp16, w.tail->cluster, s);
+}
+
+// The claim units a dataflow launch works off: all, or the part outside the tail.
+template <class T>
+sweep_args<T> outside_tail(int dir, const sweep_args<T>& w) {
+    sweep_args<T> a = w;
+    if (w.tail) {
+        if (dir == 0) {
+            a.n_chunks = w.tail->chunk;
+        } else {
+            a.chunk = w.chunk + w.tail->chunk;
+            a.n_chunks = w.n_chunks - w.tail->chunk;
+        }
+    }
+    return a;
+}
+
 template <class F>
-void set_smem(F* kernel, size_t bytes) {
-    if (bytes > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+int clusters_of(F* kernel, int size) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTailSmem)) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(size));
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = kTailSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = static_cast<unsigned>(size);
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
 }
 
 template <int K>
-void seg32(const sweep_args<float>& a, const double* in64, cudaStream_t s) {
-    const size_t smem = static_cast<size_t>(a.seg_rows) * K * sizeof(float);
-    set_smem(k_seg32<K>, smem);
-    k_seg32<K><<<1, kSegThreads, smem, s>>>(a, in64);
-}
-
-template <int K>
-void sweep32_dir(int dir, const sweep_args<float>& a, const double* in64, int grid, cudaStream_t s) {
-    if (dir == 1 && a.seg_rows) seg32<K>(a, in64, s);
-    if (a.n_items) {
+void sweep32_dir(int dir, const sweep_args<float>& w, const double* in64, int grid, cudaStream_t s) {
+    const sweep_args<float> a = outside_tail(dir, w);
+    if (dir == 1 && w.tail) tail32(dir, w, in64, false, s);
+    if (a.n_items && a.n_chunks) {
         if (a.val16) {
             if (dir == 0) k_df32<0, K, true><<<grid, kSweepThreads, 0, s>>>(a, in64);
             else          k_df32<1, K, true><<<grid, kSweepThreads, 0, s>>>(a, in64);
@@ -1011,19 +1612,29 @@ void sweep32_dir(int dir, const sweep_args<float>& a, const double* in64, int gr
             else          k_df32<1, K, false><<<grid, kSweepThreads, 0, s>>>(a, in64);
         }
     }
-    if (dir == 0 && a.seg_rows) seg32<K>(a, in64, s);
+    if (dir == 0 && w.tail) tail32(dir, w, in64, false, s);
 }
 
 }  // namespace
 
-void launch_sweep64(int dir, const sweep_args<double>& a, int grid, cudaStream_t s) {
-    const size_t smem = static_cast<size_t>(a.seg_rows) * sizeof(double);
-    if (dir == 1 && a.seg_rows) { set_smem(k_seg64, smem); k_seg64<<<1, kSegThreads, smem, s>>>(a); }
-    if (a.n_items) {
+int tail_cluster_size() {
+    for (int size : {16, 8}) {
+        const int n = std::min({clusters_of(k_tail64, size), clusters_of(k_tail32<1, false>, size), clusters_of(k_tail32<1, true>, size),
+                                clusters_of(k_tail32<2, false>, size), clusters_of(k_tail32<2, true>, size),
+                                clusters_of(k_tail32<4, false>, size), clusters_of(k_tail32<4, true>, size)});
+        if (n > 0) return size;
+    }
+    return 0;
+}
+
+void launch_sweep64(int dir, const sweep_args<double>& w, int grid, cudaStream_t s) {
+    const sweep_args<double> a = outside_tail(dir, w);
+    if (dir == 1 && w.tail) tail64(dir, w, s);
+    if (a.n_items && a.n_chunks) {
         if (dir == 0) k_df64<0><<<grid, kSweepThreads, 0, s>>>(a);
         else          k_df64<1><<<grid, kSweepThreads, 0, s>>>(a);
     }
-    if (dir == 0 && a.seg_rows) { set_smem(k_seg64, smem); k_seg64<<<1, kSegThreads, smem, s>>>(a); }
+    if (dir == 0 && w.tail) tail64(dir, w, s);
 }
 
 void launch_sweep32(int dir, const sweep_args<float>& a, int grid, cudaStream_t s) {
@@ -1049,15 +1660,19 @@ int sweep_grid64(int num_sms) {
 }
 
 template <int K>
-void sweep32_batch_dir(int dir, const sweep_args<float>& a, int grid, cudaStream_t s) {
-    if (!a.n_items) return;
-    if (a.val16) {
-        if (dir == 0) k_dw32<0, K, true><<<grid, kSweepThreads, 0, s>>>(a);
-        else          k_dw32<1, K, true><<<grid, kSweepThreads, 0, s>>>(a);
-    } else {
-        if (dir == 0) k_dw32<0, K, false><<<grid, kSweepThreads, 0, s>>>(a);
-        else          k_dw32<1, K, false><<<grid, kSweepThreads, 0, s>>>(a);
+void sweep32_batch_dir(int dir, const sweep_args<float>& w, int grid, cudaStream_t s) {
+    const sweep_args<float> a = outside_tail(dir, w);
+    if (dir == 1 && w.tail) tail32(dir, w, nullptr, true, s);
+    if (a.n_items && a.n_chunks) {
+        if (a.val16) {
+            if (dir == 0) k_dw32<0, K, true><<<grid, kSweepThreads, 0, s>>>(a);
+            else          k_dw32<1, K, true><<<grid, kSweepThreads, 0, s>>>(a);
+        } else {
+            if (dir == 0) k_dw32<0, K, false><<<grid, kSweepThreads, 0, s>>>(a);
+            else          k_dw32<1, K, false><<<grid, kSweepThreads, 0, s>>>(a);
+        }
     }
+    if (dir == 0 && w.tail) tail32(dir, w, nullptr, true, s);
 }
 
 void launch_sweep32_batch(int dir, const sweep_args<float>& a, int grid, cudaStream_t s) {
