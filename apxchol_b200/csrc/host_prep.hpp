@@ -233,7 +233,10 @@ void index_levels(sweep_plan& p, int32_t n_levels);
 
 // The cluster tail of a factor: the longest run of last levels (row ranges) of
 // at most tail_level_rows rows each and max_rows together; none below
-// kTailMinLevels levels (a launch costs about as much as two levels save).
+// kTailMinLevels levels (too few to pay for a launch). Wider levels have work
+// for more SMs than a cluster's: pairs at limits of 256 / 512 / 1024 / 2048 rows,
+// us: 128^3 fp32 628 / 622 / 645 / 701, fp64 858 / 870 / 900 / 940; 61^3 fp32
+// 234 / 219 / 214 / 224; 6-regular n = 100003 fp32 603 / 578 / 571 / 578.
 struct tail_span {
     int32_t level = 0;        // its first forward level; backward it is the first fwd_levels - level levels
     uint32_t first = 0, rows = 0;
