@@ -108,25 +108,29 @@ __device__ __forceinline__ double dadd4(double a, double b, double c, double d) 
 // a / d correctly rounded for a divisor known before a, in two dependent
 // operations: with 1 / d = h + l (l the rounded remainder of h = RN(1 / d), so
 // the pair is within 2^-104), RN(a h + RN(a l)) differs from a / d by less than
-// 2^-103 of it before its one rounding. d is an fp32 value: a / d lies at least
-// 2^-79 of itself away from every midpoint of two doubles (a - m d is a nonzero
-// whole multiple of the unit of the 54-bit m times the 24-bit d; it is not zero
-// since m d has more than 53 bits), so the rounding is that of a / d. Operands
-// near overflow or underflow divide. fp64 operations take about 40 cycles each
-// on the row's critical path here (a divide about nine of them).
+// 2^-103 of it, and by at most another 2^-1075 where a l is subnormal, before
+// its one rounding. d is an fp32 value: a / d lies at least 2^-79 of itself away
+// from every midpoint of two doubles (a - m d is a nonzero whole multiple of the
+// unit of the 54-bit m times the 24-bit d; it is not zero since m d has more than
+// 53 bits), so the rounding is that of a / d. The short way is taken for
+// 2^-120 <= |d| < 2^120 and 2^-831 <= |a| < 2^850: the quotient lies in
+// (2^-951, 2^970), where 2^-1075 is below 2^-123 of it (down to 2^-995 it is
+// below the 2^-80 that the midpoints leave) and nothing overflows. Other
+// operands divide. fp64 operations take about 40 cycles each on the row's
+// critical path here (a divide about nine of them).
 struct recip64 {
     double d, h, l;
-    unsigned span;   // exponents of a that take the short way: [123, 123 + span)
+    unsigned span;   // biased exponents of a that take the short way: [192, 192 + span)
     __device__ __forceinline__ double quotient(double a) const {
         double q = __fma_rn(a, h, __dmul_rn(a, l));
-        if (((static_cast<unsigned>(__double2hiint(a)) >> 20) & 0x7ffu) - 123u >= span) q = __ddiv_rn(a, d);
+        if (((static_cast<unsigned>(__double2hiint(a)) >> 20) & 0x7ffu) - 192u >= span) q = __ddiv_rn(a, d);
         return q;
     }
 };
 __device__ __forceinline__ recip64 recip_of(double d) {
     const double h = __drcp_rn(d);
     const unsigned ed = (static_cast<unsigned>(__double2hiint(d)) >> 20) & 0x7ffu;
-    return {d, h, __dmul_rn(__fma_rn(-d, h, 1.0), h), ed - (1023u - 120u) < 240u ? 1750u : 0u};
+    return {d, h, __dmul_rn(__fma_rn(-d, h, 1.0), h), ed - (1023u - 120u) < 240u ? 1681u : 0u};
 }
 
 // ---------------------------------------------------------------------------
