@@ -641,49 +641,63 @@ __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const do
     }
 }
 
-// a / d in fp32, correctly rounded, for a divisor known before the dividend: a
-// Newton step on a r, r = RN(1 / d), makes the quotient faithful, and a faithful
-// quotient corrected by its exact remainder times r is the rounded one
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990). Divisors and dividends whose reciprocal, quotient or
-// remainder leaves the normal range divide.
-struct recip32 {
-    float d, r;
-    unsigned span;   // exponents of a that take the short way: [67, 67 + span)
-    __device__ __forceinline__ float quotient(float a) const {
-        float q = __fmul_rn(a, r);
-        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
-        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
-        if (((__float_as_uint(a) >> 23) & 0xffu) - 67u >= span) q = __fdiv_rn(a, d);
-        return q;
+// Sums a lane's nk operand rows (at most B, loaded once into yv) into acc in
+// order, oldest dependency first, polling for those still to come. Returns false
+// when the warp must drain. Which polls are cheapest depends on the row's width:
+//  * up to 2 columns, straight-line code with one vote a pass and the sums behind
+//    the last pass: a pass over the pending rows is what stands between the last
+//    operand's arrival and the row;
+//  * from 4 columns on a lane consumes its rows as they arrive and polls only
+//    those from the first missing one on (a poll of 16 bytes and more costs what
+//    the vote saves), by predicate at 4 columns and by branch from 8 on.
+// One pair of sweeps, all levels in the dataflow launches, us, straight line ->
+// this rule, mean of seven placements of the factor: R-MAT-14 k = 4 777 -> 734,
+// k = 8 1101 -> 887, k = 16 1807 -> 1532; 6-regular n = 100003 1641 -> 1563,
+// 2288 -> 1880, 3793 -> 3307; 96^3 grid 671 -> 630, 934 -> 803, 1401 -> 1314.
+// At one column in order against straight line: 758 : 724, 2204 : 2125, 754 : 732.
+template <int B, int K>
+__device__ __forceinline__ bool gather32(const sweep_args<float>& a, int where, uint32_t row, idle_clock& clk, uint32_t nk,
+                                         const uint32_t (&jj)[B], const float (&ww)[B], float (&yv)[B][K], float (&acc)[K]) {
+    if constexpr (K <= 2) {
+        for (;;) {
+            bool open = false;
+#pragma unroll
+            for (int k = 0; k < B; ++k) open |= static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
+            if (!__any_sync(kFull, open)) break;
+            if (clk.idle(a.err, a.budget_ns, where, row)) return false;
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                ld_row_if<K>(static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]), a.out + static_cast<size_t>(jj[k]) * K, yv[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+            if (static_cast<uint32_t>(k) < nk)
+#pragma unroll
+                for (int r = 0; r < K; ++r) acc[r] = __fmaf_rn(ww[k], yv[k][r], acc[r]);
+    } else {
+        uint32_t kpos = 0;
+        for (;;) {
+            const uint32_t before = kpos;
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                if (kpos == static_cast<uint32_t>(k) && kpos < nk && row_ready<K>(yv[k])) {
+#pragma unroll
+                    for (int r = 0; r < K; ++r) acc[r] = __fmaf_rn(ww[k], yv[k][r], acc[r]);
+                    ++kpos;
+                }
+            }
+            if (__all_sync(kFull, kpos >= nk)) break;
+            if (__any_sync(kFull, kpos != before)) clk.spins = 0;
+            else if (clk.idle(a.err, a.budget_ns, where, row)) return false;
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const bool on = static_cast<uint32_t>(k) >= kpos && static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
+                const float* p = a.out + static_cast<size_t>(jj[k]) * K;
+                if constexpr (K == 4) ld_row_if<K>(on, p, yv[k]);
+                else if (on) ld_row<K>(p, yv[k]);
+            }
+        }
     }
-};
-__device__ __forceinline__ recip32 recip_of(float d) {
-    return {d, __frcp_rn(d), ((__float_as_uint(d) >> 23) & 0xffu) - (127u - 40u) < 80u ? 120u : 0u};
-}
-
-// Sums nk operand rows into acc in order once the warp has all of them (oldest
-// dependency first): ld(on, j, y) loads operand row j into y where on. Straight
-// line code with one vote a pass, since a pass over the pending rows is what
-// stands between the last operand's arrival and the row. Narrow rows wait on
-// the newest pending one (see kLight). Returns false when the warp must drain.
-template <int B, int K, class Ld, class Idle>
-__device__ __forceinline__ bool gather32(uint32_t nk, const uint32_t (&jj)[B], const float (&ww)[B], float (&yv)[B][K],
-                                         float (&acc)[K], Ld&& ld, Idle&& idle) {
-    for (;;) {
-        bool open = false;
-#pragma unroll
-        for (int k = 0; k < B; ++k) open |= static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
-        if (!__any_sync(kFull, open)) break;
-        if (idle()) return false;
-#pragma unroll
-        for (int k = 0; k < B; ++k) ld(static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]), jj[k], yv[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < B; ++k)
-        if (static_cast<uint32_t>(k) < nk)
-#pragma unroll
-            for (int r = 0; r < K; ++r) acc[r] = __fmaf_rn(ww[k], yv[k][r], acc[r]);
     return true;
 }
 
@@ -697,7 +711,6 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
     float acc[K];
 #pragma unroll
     for (int r = 0; r < K; ++r) acc[r] = 0.0f;
-    const recip32 inv = recip_of(s.d);
     idle_clock clk;
     for (uint32_t jb = 0; jb < Jmax; jb += B) {
         if (jb > 0) {
@@ -715,14 +728,13 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
         const uint32_t t0 = (jb << v.lg) + v.u;
         const uint32_t nk = t0 < v.len ? min(static_cast<uint32_t>(B), ((v.len - t0 - 1u) >> v.lg) + 1u) : 0u;
         float yv[B][K];
-        const auto ld = [&](bool on, uint32_t j, float (&y)[K]) { ld_row_if<K>(on, a.out + static_cast<size_t>(j) * K, y); };
 #pragma unroll
         for (int k = 0; k < B; ++k) {
 #pragma unroll
             for (int r = 0; r < K; ++r) yv[k][r] = 0.0f;
-            ld(static_cast<uint32_t>(k) < nk, s.jj[k], yv[k]);
+            ld_row_if<K>(static_cast<uint32_t>(k) < nk, a.out + static_cast<size_t>(s.jj[k]) * K, yv[k]);
         }
-        if (!gather32<B, K>(nk, s.jj, s.ww, yv, acc, ld, [&] { return clk.idle(a.err, a.budget_ns, where, v.row); })) return false;
+        if (!gather32<B, K>(a, where, v.row, clk, nk, s.jj, s.ww, yv, acc)) return false;
         clk.spins = 0;
     }
     // fixed butterfly over the group's lanes
@@ -730,9 +742,11 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
 #pragma unroll
         for (int r = 0; r < K; ++r) acc[r] += __shfl_xor_sync(kFull, acc[r], static_cast<int>(o), static_cast<int>(v.G));
     if (v.valid && v.u == 0) {
+        // a plain division: a reciprocal formed before the wait (recip32) was slower here, where other warps
+        // hide it (k = 1, us: R-MAT-16 2184 : 2213, 96^3 grid 709 : 732)
         float y[K];
 #pragma unroll
-        for (int r = 0; r < K; ++r) y[r] = inv.quotient(s.rhs[r] - acc[r]);
+        for (int r = 0; r < K; ++r) y[r] = __fdiv_rn(s.rhs[r] - acc[r], s.d);
         st_row<K>(a.out + static_cast<size_t>(v.row) * K, y);
         if (a.reset) {   // re-arm after the right-hand side was consumed (see run64)
             float sent[K];
@@ -1289,6 +1303,27 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail64(const tail_args<doub
 
 // ---- fp32: KC columns of the k per cluster, every lane adding its entries in
 // order (oldest dependency first), the lanes' sums by a fixed butterfly
+
+// a / d in fp32, correctly rounded, for a divisor known before the dividend: a
+// Newton step on a r, r = RN(1 / d), makes the quotient faithful, and a faithful
+// quotient corrected by its exact remainder times r is the rounded one
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990). Divisors and dividends whose reciprocal, quotient or
+// remainder leaves the normal range divide.
+struct recip32 {
+    float d, r;
+    unsigned span;   // exponents of a that take the short way: [67, 67 + span)
+    __device__ __forceinline__ float quotient(float a) const {
+        float q = __fmul_rn(a, r);
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), r, q);
+        if (((__float_as_uint(a) >> 23) & 0xffu) - 67u >= span) q = __fdiv_rn(a, d);
+        return q;
+    }
+};
+__device__ __forceinline__ recip32 recip_of(float d) {
+    return {d, __frcp_rn(d), ((__float_as_uint(d) >> 23) & 0xffu) - (127u - 40u) < 80u ? 120u : 0u};
+}
 
 template <int KC>
 struct near_row32 {
