@@ -61,35 +61,62 @@ __device__ __forceinline__ unsigned backoff_ns(int spins) {
     return spins < 4 ? 0u : min(16u << min((spins - 4) >> 1, 3), 128u);
 }
 
-// Warp-uniform check of the error word and the time budget. Returns true when
-// the warp must drain (budget exhausted -> error raised, or another warp failed).
-__device__ __forceinline__ bool wait_must_stop(dev_error* err, unsigned long long t0, unsigned long long budget,
-                                               int where, uint32_t row) {
-    int stop = 0;
-    if ((threadIdx.x & 31) == 0) {
-        if (ld_relaxed_int(&err->code) != 0) {
-            stop = 1;
-        } else if (globaltimer() - t0 > budget) {
-            raise_error(err, -4 /* APXB_ERR_TIMEOUT */, where, row);
-            stop = 1;
-        }
-    }
-    return __shfl_sync(kFull, stop, 0) != 0;
+// Warp-uniform look at the error word and the time budget: another warp has
+// failed, the budget is over, or neither.
+enum wait_state : int { kWait = 0, kFailed = 1, kOver = 2 };
+__device__ __forceinline__ int look(dev_error* err, unsigned long long t0, unsigned long long budget) {
+    int st = kWait;
+    if ((threadIdx.x & 31) == 0)
+        st = ld_relaxed_int(&err->code) != 0 ? kFailed : (globaltimer() - t0 > budget ? kOver : kWait);
+    return __shfl_sync(kFull, st, 0);
+}
+__device__ __forceinline__ bool run_out(dev_error* err, int where, uint32_t row) {
+    if ((threadIdx.x & 31) == 0) raise_error(err, -4 /* APXB_ERR_TIMEOUT */, where, row);
+    return true;
 }
 
-// Idle bookkeeping of a warp-uniform polling loop; returns true to drain.
+// Idle bookkeeping of a warp-uniform polling loop; returns true to drain. The
+// budget limits the time without progress. A loop clears spins when an operand
+// has come in, or tells when the budget is over whether its lanes wait for other
+// operands than the last time it was over (moved()): then the budget starts anew,
+// so such a wait ends between one and two budgets after its last operand. What
+// the lanes waited for lies in shared memory, since a register for it cost the
+// loops 1 to 8 % (fp64, R-MAT-14 in dataflow launches alone, 961 : 1036 us).
+__device__ __forceinline__ unsigned long long& last_pending() {
+    __shared__ unsigned long long words[kSweepThreads];
+    return words[threadIdx.x];
+}
+
 struct idle_clock {
     int spins = 0;
     unsigned long long t0 = 0;
-    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row) {
+    template <class Moved>
+    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row, Moved&& moved) {
         if (spins == 0 && (threadIdx.x & 31) == 0) t0 = globaltimer();
         ++spins;
-        if ((spins & 15) == 0 && wait_must_stop(err, __shfl_sync(kFull, t0, 0), budget, where, row)) return true;
+        if ((spins & 15) == 0) {
+            const int st = look(err, __shfl_sync(kFull, t0, 0), budget);
+            if (st == kFailed) return true;
+            if (st == kOver) {
+                if (!moved(row)) return run_out(err, where, row);
+                if ((threadIdx.x & 31) == 0) t0 = globaltimer();
+            }
+        }
         const unsigned ns = backoff_ns(spins);
         if (ns) __nanosleep(ns);
         return false;
     }
+    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row) {
+        return idle(err, budget, where, row, [](uint32_t) { return false; });
+    }
 };
+// Warp-uniform: some lane waits for other operands than at the last call.
+__device__ __forceinline__ bool pending_changed(uint32_t row, uint32_t batch, unsigned mask) {
+    const unsigned long long now = static_cast<unsigned long long>(row) << 32 | batch << 8 | mask;
+    const bool changed = __any_sync(kFull, now != last_pending());
+    last_pending() = now;
+    return changed;
+}
 
 __device__ __forceinline__ void leave(sweep_ctl* ctl) {
     if ((threadIdx.x & 31) == 0) {
@@ -292,6 +319,8 @@ struct far_src64 {
     idle_clock clk;
     __device__ __forceinline__ void load(bool on, uint32_t j, double& y) const { ld_if(on, a.out + j, y); }
     __device__ __forceinline__ bool idle(uint32_t row) { return clk.idle(a.err, a.budget_ns, where, row); }
+    template <class Moved>
+    __device__ __forceinline__ bool idle(uint32_t row, Moved&& moved) { return clk.idle(a.err, a.budget_ns, where, row, moved); }
     __device__ __forceinline__ void progress() { clk.spins = 0; }
 };
 
@@ -439,7 +468,13 @@ __device__ __forceinline__ bool run_lane64(far_src64& src, stage_data64& s, doub
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) open |= static_cast<uint32_t>(k) < n && is_sent(y[k]);
         if (!__any_sync(kFull, open)) break;
-        if (src.idle(v.row)) return false;
+        const auto moved = [&](uint32_t row) {
+            unsigned p = 0;
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) p |= static_cast<uint32_t>(k) < n && is_sent(y[k]) ? 1u << k : 0u;
+            return pending_changed(row, 0, p);
+        };
+        if (src.idle(v.row, moved)) return false;
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) src.load(static_cast<uint32_t>(k) < n && is_sent(y[k]), s.jj[k], y[k]);
     }
@@ -488,6 +523,7 @@ __device__ __forceinline__ bool run64(const sweep_args<double>& a, stage_data64&
 template <int DIR>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_df64(const sweep_args<double> a) {
     if (a.skip && *a.skip) return;
+    last_pending() = 0;
     __shared__ __align__(16) double prods[kSweepThreads / 32][32 * kBatch];
     const unsigned lane = threadIdx.x & 31u;
     double* prod = prods[threadIdx.x >> 5];
@@ -644,27 +680,33 @@ __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const do
 // Sums a lane's nk operand rows (at most B, loaded once into yv) into acc in
 // order, oldest dependency first, polling for those still to come. Returns false
 // when the warp must drain. Which polls are cheapest depends on the row's width:
-//  * up to 2 columns, straight-line code with one vote a pass and the sums behind
-//    the last pass: a pass over the pending rows is what stands between the last
+//  * one column, straight-line code with one vote a pass and the sums behind the
+//    last pass: a pass over the pending rows is what stands between the last
 //    operand's arrival and the row;
-//  * from 4 columns on a lane consumes its rows as they arrive and polls only
-//    those from the first missing one on (a poll of 16 bytes and more costs what
-//    the vote saves), by predicate at 4 columns and by branch from 8 on.
+//  * from 2 columns on a lane consumes its rows as they arrive and polls only
+//    those from the first missing one on (the wider polls cost what the vote
+//    saves), by predicate up to 4 columns and by branch from 8 on.
 // One pair of sweeps, all levels in the dataflow launches, us, straight line ->
 // this rule, mean of seven placements of the factor: R-MAT-14 k = 4 777 -> 734,
 // k = 8 1101 -> 887, k = 16 1807 -> 1532; 6-regular n = 100003 1641 -> 1563,
 // 2288 -> 1880, 3793 -> 3307; 96^3 grid 671 -> 630, 934 -> 803, 1401 -> 1314.
 // At one column in order against straight line: 758 : 724, 2204 : 2125, 754 : 732.
 template <int B, int K>
-__device__ __forceinline__ bool gather32(const sweep_args<float>& a, int where, uint32_t row, idle_clock& clk, uint32_t nk,
+__device__ __forceinline__ bool gather32(const sweep_args<float>& a, int where, uint32_t row, uint32_t batch, idle_clock& clk, uint32_t nk,
                                          const uint32_t (&jj)[B], const float (&ww)[B], float (&yv)[B][K], float (&acc)[K]) {
-    if constexpr (K <= 2) {
+    if constexpr (K == 1) {
         for (;;) {
             bool open = false;
 #pragma unroll
             for (int k = 0; k < B; ++k) open |= static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
             if (!__any_sync(kFull, open)) break;
-            if (clk.idle(a.err, a.budget_ns, where, row)) return false;
+            const auto moved = [&](uint32_t r) {
+                unsigned p = 0;
+#pragma unroll
+                for (int k = 0; k < B; ++k) p |= static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]) ? 1u << k : 0u;
+                return pending_changed(r, batch, p);
+            };
+            if (clk.idle(a.err, a.budget_ns, where, row, moved)) return false;
 #pragma unroll
             for (int k = 0; k < B; ++k)
                 ld_row_if<K>(static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]), a.out + static_cast<size_t>(jj[k]) * K, yv[k]);
@@ -693,7 +735,7 @@ __device__ __forceinline__ bool gather32(const sweep_args<float>& a, int where, 
             for (int k = 0; k < B; ++k) {
                 const bool on = static_cast<uint32_t>(k) >= kpos && static_cast<uint32_t>(k) < nk && !row_ready<K>(yv[k]);
                 const float* p = a.out + static_cast<size_t>(jj[k]) * K;
-                if constexpr (K == 4) ld_row_if<K>(on, p, yv[k]);
+                if constexpr (K <= 4) ld_row_if<K>(on, p, yv[k]);
                 else if (on) ld_row<K>(p, yv[k]);
             }
         }
@@ -734,7 +776,7 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
             for (int r = 0; r < K; ++r) yv[k][r] = 0.0f;
             ld_row_if<K>(static_cast<uint32_t>(k) < nk, a.out + static_cast<size_t>(s.jj[k]) * K, yv[k]);
         }
-        if (!gather32<B, K>(a, where, v.row, clk, nk, s.jj, s.ww, yv, acc)) return false;
+        if (!gather32<B, K>(a, where, v.row, jb / B, clk, nk, s.jj, s.ww, yv, acc)) return false;
         clk.spins = 0;
     }
     // fixed butterfly over the group's lanes
@@ -761,6 +803,7 @@ __device__ __forceinline__ bool run32(const sweep_args<float>& a, stage_data32<K
 template <int DIR, int K, bool H>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_df32(const sweep_args<float> a, const double* in64) {
     if (a.skip && *a.skip) return;
+    last_pending() = 0;
     const unsigned lane = threadIdx.x & 31u;
     chunk_claim cc;
     cc.start(a);
@@ -1036,14 +1079,25 @@ __device__ __forceinline__ void peer_st_row(unsigned p, const float (&y)[KC]) {
 }
 
 // Polls of shared memory disturb no other SM and the loop around them has to be
-// short: the error word and the time budget are looked at every 4096th poll.
+// short: the error word and the time budget are looked at every 4096th poll, as
+// in idle_clock.
 struct near_clock {
-    unsigned spins = 0;
+    unsigned spins = 0, seen = 0;
     unsigned long long t0 = 0;
-    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row) {
+    template <class Pending>
+    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row, Pending&& pending) {
         if ((++spins & 4095u) != 0) return false;
         if (t0 == 0) t0 = globaltimer();
-        return wait_must_stop(err, __shfl_sync(kFull, t0, 0), budget, where, row);
+        const int st = look(err, __shfl_sync(kFull, t0, 0), budget);
+        if (st == kWait) return false;
+        const unsigned now = pending();
+        if (st == kFailed || !__any_sync(kFull, now != seen)) return st == kFailed || run_out(err, where, row);
+        seen = now;
+        t0 = globaltimer();
+        return false;
+    }
+    __device__ __forceinline__ bool idle(dev_error* err, unsigned long long budget, int where, uint32_t row) {
+        return idle(err, budget, where, row, [this] { return seen; });
     }
 };
 
@@ -1151,8 +1205,9 @@ __device__ __forceinline__ void near_outside64(const tail_args<double>& a, const
 template <int NB>
 __device__ __forceinline__ bool near_batch64(const tail_args<double>& a, const tail_seat& t, const near_row64& s,
                                              double (&y)[kBatch], uint32_t jb, uint32_t gend, int where, double* prod,
-                                             uint32_t& at, double& sum, near_clock& clk) {
+                                             uint32_t& at, double& sum) {
     const lane_view& v = s.v;
+    near_clock clk;
     const unsigned lane = threadIdx.x & 31u;
     const double* pr = prod + v.G * v.gid;
     const unsigned W = v.thin ? 4u : 1u, c = v.thin ? (v.u & 3u) : 0u;
@@ -1212,18 +1267,17 @@ __device__ __forceinline__ bool near_group64(const tail_args<double>& a, const t
     const uint32_t gend = v.thin ? (v.len & ~3u) : v.len;   // entries the chains take
     double sum = 0.0;
     uint32_t at = 0, jb = 0;
-    near_clock clk;
     for (; jb + kBatch < Jmax; jb += kBatch) {
-        if (!near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum, clk)) return false;
+        if (!near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum)) return false;
         near_entries64(a, v, jb + kBatch, s);
         near_outside64(a, s, y);
         __syncwarp();   // the batch's products have been read
     }
     const uint32_t nb = Jmax - jb;
-    const bool ok = nb <= 1 ? near_batch64<1>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
-                  : nb <= 2 ? near_batch64<2>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
-                  : nb <= 4 ? near_batch64<4>(a, t, s, y, jb, gend, where, prod, at, sum, clk)
-                            : near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum, clk);
+    const bool ok = nb <= 1 ? near_batch64<1>(a, t, s, y, jb, gend, where, prod, at, sum)
+                  : nb <= 2 ? near_batch64<2>(a, t, s, y, jb, gend, where, prod, at, sum)
+                  : nb <= 4 ? near_batch64<4>(a, t, s, y, jb, gend, where, prod, at, sum)
+                            : near_batch64<kBatch>(a, t, s, y, jb, gend, where, prod, at, sum);
     if (!ok) return false;
     if (v.thin) {   // (s0 + s1) + (s2 + s3), then the <= 3 entries left (in the row's last batch)
         sum = __dadd_rn(sum, __shfl_xor_sync(kFull, sum, 1));
@@ -1248,7 +1302,13 @@ __device__ __forceinline__ bool near_lane64(const tail_args<double>& a, const ta
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) open |= is_sent(y[k]);
         if (!__any_sync(kFull, open)) break;
-        if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
+        const auto pending = [&] {
+            unsigned p = 0;
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) p |= is_sent(y[k]) ? 1u << k : 0u;
+            return p;
+        };
+        if (clk.idle(a.err, a.budget_ns, where, v.row, pending)) return false;
     }
     double p[kBatch];
 #pragma unroll
@@ -1420,7 +1480,8 @@ __device__ __forceinline__ void near_outside32(const tail_args<float>& a, const 
 // operand is in, then the sums in straight line.
 template <int KC, int NB>
 __device__ __forceinline__ bool near_batch32(const tail_args<float>& a, const tail_seat& t, const near_row32<KC>& s,
-                                             float (&yv)[kBatch][KC], int where, float (&acc)[KC], near_clock& clk) {
+                                             float (&yv)[kBatch][KC], int where, float (&acc)[KC]) {
+    near_clock clk;
     for (;;) {
         bool open = false;
 #pragma unroll
@@ -1429,7 +1490,13 @@ __device__ __forceinline__ bool near_batch32(const tail_args<float>& a, const ta
 #pragma unroll
         for (int k = 0; k < NB; ++k) open |= !row_ready<KC>(yv[k]);
         if (!__any_sync(kFull, open)) break;
-        if (clk.idle(a.err, a.budget_ns, where, s.v.row)) return false;
+        const auto pending = [&] {
+            unsigned p = 0;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) p |= !row_ready<KC>(yv[k]) ? 1u << k : 0u;
+            return p;
+        };
+        if (clk.idle(a.err, a.budget_ns, where, s.v.row, pending)) return false;
     }
 #pragma unroll
     for (int k = 0; k < NB; ++k)
@@ -1445,18 +1512,17 @@ __device__ __forceinline__ bool near_run32(const tail_args<float>& a, const tail
     const uint32_t Jmax = __reduce_max_sync(kFull, (v.len + v.G - 1u) >> v.lg);
 #pragma unroll
     for (int r = 0; r < KC; ++r) acc[r] = 0.0f;
-    near_clock clk;
     uint32_t jb = 0;
     for (; jb + kBatch < Jmax; jb += kBatch) {
-        if (!near_batch32<KC, kBatch>(a, t, s, yv, where, acc, clk)) return false;
+        if (!near_batch32<KC, kBatch>(a, t, s, yv, where, acc)) return false;
         near_entries32<KC, H>(a, v, jb + kBatch, back && !a.wide, s);
         near_outside32<KC>(a, t, s, yv);
     }
     const uint32_t nb = Jmax - jb;
-    const bool ok = nb <= 1 ? near_batch32<KC, 1>(a, t, s, yv, where, acc, clk)
-                  : nb <= 2 ? near_batch32<KC, 2>(a, t, s, yv, where, acc, clk)
-                  : nb <= 4 ? near_batch32<KC, 4>(a, t, s, yv, where, acc, clk)
-                            : near_batch32<KC, kBatch>(a, t, s, yv, where, acc, clk);
+    const bool ok = nb <= 1 ? near_batch32<KC, 1>(a, t, s, yv, where, acc)
+                  : nb <= 2 ? near_batch32<KC, 2>(a, t, s, yv, where, acc)
+                  : nb <= 4 ? near_batch32<KC, 4>(a, t, s, yv, where, acc)
+                            : near_batch32<KC, kBatch>(a, t, s, yv, where, acc);
     if (!ok) return false;
 #pragma unroll
     for (unsigned i = 5; i-- > 0;)

@@ -99,7 +99,9 @@ int apxb_engine_destroy(apxb_engine* e);
 int apxb_engine_sync(apxb_engine* e);
 /* The engine's CUDA stream (cudaStream_t), for callers that order their own work around it. */
 void* apxb_engine_stream(apxb_engine* e);
-/* Spin budget of every device wait, in nanoseconds (default 2e9). */
+/* Spin budget of every device wait, in nanoseconds (default 2e9): a wait that
+ * sees none of its operands arrive for that long ends in APXB_ERR_TIMEOUT, up
+ * to one more budget later (cluster tails look every few hundred microseconds). */
 int apxb_engine_set_spin_budget(apxb_engine* e, uint64_t ns);
 /* Blocks of the persistent sweep launches (0 = the resident grid). Any value
  * gives the same bytes; tests use it to show the result is schedule-free.
