@@ -3,6 +3,7 @@
 // negative status with the message in apxb_last_error().
 #include "apxb200.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -1065,6 +1066,38 @@ extern "C" int apxb_test_stalled_sweep(apxb_engine* e, apxb_factor* f, uint64_t 
     APXB_CK(cudaStreamSynchronize(s));
     if (rc) { disarm(f); return rc; }
     rc = finish(f);
+    disarm(f);
+    return rc;
+}
+
+extern "C" int apxb_test_stalled_launch(apxb_engine* e, apxb_factor* f, int dir, int k, int tail, uint64_t budget_ns) {
+    if (!e || !f || f->e != e || budget_ns == 0 || (dir != 0 && dir != 1)) return fail(APXB_ERR_INVALID, "bad argument");
+    const bool fp64 = f->precision == APXB_PREC_FP64;
+    if (fp64 ? k != 1 : (k != 1 && k != 2 && k != 4 && k != 8 && k != 16)) return fail(APXB_ERR_INVALID, "bad k");
+    apxb::tail_plan& t = f->tail[dir][fp64 ? 0 : 1];
+    const apxb::tail_plan whole = t;
+    const auto& first = (dir == 0 ? f->h.fwd_plan : f->h.bck_plan).level_item;
+    const uint32_t left_units = t.rows ? (dir == 0 ? t.chunk : f->n_chunks[dir] - t.chunk) : f->n_chunks[dir];
+    if (tail ? !t.rows : left_units < 2) return fail(APXB_ERR_INVALID, "the direction has no such launch");
+    APXB_CK(cudaSetDevice(e->device));
+    cudaStream_t s = e->stream;
+    int rc = e->ensure_stage(static_cast<size_t>(f->h.n) * k);
+    if (rc) return rc;
+    const size_t mk = static_cast<size_t>(f->h.m) * k;
+    APXB_CK(cudaMemsetAsync(e->d_stage_a, 0, 8 * mk, s));
+    if (tail) {
+        t.item0 = *std::upper_bound(first.begin(), first.end(), t.item0);   // past the tail's first level
+    } else {
+        const apxb::sweep_ctl start{1u, 0u};   // past claim unit 0
+        APXB_CK(cudaMemcpyAsync(f->ctl + dir, &start, sizeof(start), cudaMemcpyHostToDevice, s));
+    }
+    const unsigned long long saved = e->budget_ns;
+    e->budget_ns = budget_ns;
+    rc = fp64 ? pair_fp64(f, e->d_stage_a, e->d_stage_b) : pair_fp32(f, k, e->d_stage_a, e->d_stage_b);
+    e->budget_ns = saved;
+    t = whole;
+    APXB_CK(cudaStreamSynchronize(s));
+    if (!rc) rc = e->take_error();
     disarm(f);
     return rc;
 }

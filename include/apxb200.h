@@ -323,6 +323,11 @@ int apxb_batch_sweep_timed(apxb_batch* b, int reps, double* fwd_seconds, double*
  * engine usable. Used by the tests to show a stalled wait ends in an error,
  * not a hang. */
 int apxb_test_stalled_sweep(apxb_engine* e, apxb_factor* f, uint64_t budget_ns);
+/* The same for one launch of a pair of sweeps as the callers' sweeps run it (k
+ * columns for fp32 / fp16 factors): direction dir's cluster tail without its
+ * first level (tail != 0), or its dataflow launch without its first claim unit.
+ * APXB_ERR_INVALID when the direction has no such launch. */
+int apxb_test_stalled_launch(apxb_engine* e, apxb_factor* f, int dir, int k, int tail, uint64_t budget_ns);
 
 /* ---- device preparation test hook ----
  * apxb_factor_create prepares factors with round sizes and fp32 / fp64
