@@ -971,6 +971,7 @@ std::string same_plan(const char* dir, const dev_plan_out& o, const sweep_plan& 
     if (!(e = same((p + "idx").c_str(), o.idx, pl.idx, o.n_entries, s)).empty()) return e;
     if (!(e = same((p + "val").c_str(), o.val, pl.val, o.n_entries, s)).empty()) return e;
     if (!(e = same((p + "chunk").c_str(), o.chunk, pl.chunk, static_cast<size_t>(o.n_chunks) + 1, s)).empty()) return e;
+    if (o.level_item != pl.level_item || o.level_chunk != pl.level_chunk) return p + "level tables differ";
     return {};
 }
 
@@ -1004,11 +1005,14 @@ extern "C" int apxb_test_prep_compare(apxb_engine* e, uint32_t n, const uint32_t
         if (h.m != hf.m || h.nnz_factor != hf.nnz_factor || h.nnz_stored != hf.nnz_stored || h.dropped != hf.dropped ||
             h.dropped_flush != hf.dropped_flush || h.fwd_levels != hf.fwd_levels || h.bck_levels != hf.bck_levels)
             return fail(APXB_ERR_INVALID, "sizes or counts differ");
+        if (h.level_bound != hf.level_bound) return fail(APXB_ERR_INVALID, "level bounds differ");
         for (int dir = 0; dir < 2 && why.empty(); ++dir) {
             apxb::dev_plan_out o;
             o.n_items = (dir == 0 ? h.fwd_plan : h.bck_plan).n_items;
             o.info = f.info[dir]; o.ord = f.ord[dir]; o.ptr = f.ptr[dir]; o.idx = f.idx[dir]; o.val = f.val[dir];
             o.chunk = f.chunk[dir]; o.n_chunks = f.n_chunks[dir];
+            o.level_item = (dir == 0 ? h.fwd_plan : h.bck_plan).level_item;
+            o.level_chunk = (dir == 0 ? h.fwd_plan : h.bck_plan).level_chunk;
             o.n_entries = (dir == 0 ? hf.fwd_plan : hf.bck_plan).idx.size();
             why = apxb::same_plan(dir == 0 ? "forward plan" : "backward plan", o, dir == 0 ? hf.fwd_plan : hf.bck_plan, s);
         }

@@ -53,9 +53,6 @@ std::vector<uint32_t> column_ranges(const P* ptr, uint32_t cols, unsigned T) {
     return jb;
 }
 
-// Plan of one direction (see sweep_plan). level[r] = level of row r in this
-// direction; (ptr, idx, val) = the canonical arrays of the direction (forward:
-// CSR(L11), diagonal last; backward: CSC(L11), diagonal first).
 // Rows grouped by (level, class): levels ascending, classes 0..n_cls-1, rows
 // ascending inside a group -- one stable counting sort. cls[r] == n_cls leaves
 // row r out. start[l * n_cls + c] is where group (l, c) begins in rows.
@@ -72,6 +69,9 @@ void group_rows(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels,
         if (cls[r] < n_cls) rows[cur[static_cast<size_t>(level[r]) * n_cls + cls[r]]++] = r;
 }
 
+// Plan of one direction (see sweep_plan). level[r] = level of row r in this
+// direction; (ptr, idx, val) = the canonical arrays of the direction (forward:
+// CSR(L11), diagonal last; backward: CSC(L11), diagonal first).
 // val16 (fp16 storage, nullable): binary16 values beside val, re-laid the
 // same way into plan.val16.
 void build_plan(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels, const std::vector<uint32_t>& bits,
@@ -146,6 +146,21 @@ void build_plan(uint32_t m, const std::vector<int32_t>& level, int32_t n_levels,
     index_levels(plan, n_levels);
 }
 
+// The level tables (index_levels): ascending, from the first item and claim unit
+// to the ends, and every item between its level's bounds. A sweep leaves the
+// items behind one of these bounds to its cluster tail.
+std::string check_levels(const sweep_plan& pl) {
+    const auto &li = pl.level_item, &lc = pl.level_chunk;
+    if (li.size() < 2 || lc.size() != li.size() || pl.item_level.size() != pl.n_items || pl.chunk.empty()) return "bad level table sizes";
+    if (li.front() != 0 || li.back() != pl.n_items || lc.front() != 0 || lc.back() + 1 != pl.chunk.size()) return "bad level table ends";
+    for (size_t l = 0; l + 1 < li.size(); ++l) {
+        if (li[l] > li[l + 1] || lc[l] > lc[l + 1] || pl.chunk[lc[l]] != li[l]) return "bad level bounds";
+        for (uint32_t c = li[l]; c < li[l + 1]; ++c)
+            if (pl.item_level[c] != static_cast<int32_t>(l)) return "item outside its level's bounds";
+    }
+    return {};
+}
+
 // Plan invariants the kernels rely on (checked at every setup): every row is
 // in exactly one slot; items hold 1..32/G rows of one level, in nondecreasing
 // level order; every slot's entries end with its own diagonal.
@@ -177,7 +192,7 @@ std::string check_plan(uint32_t m, const std::vector<int32_t>& level, const swee
     if (pl.chunk.empty() || pl.chunk.front() != 0 || pl.chunk.back() != pl.n_items) return "bad chunk table";
     for (size_t i = 0; i + 1 < pl.chunk.size(); ++i)
         if (pl.chunk[i + 1] <= pl.chunk[i] || pl.chunk[i + 1] - pl.chunk[i] > 8) return "bad chunk";
-    return {};
+    return check_levels(pl);
 }
 
 // APXB_PREP_TRACE=1: the time of each preparation stage on stderr.
@@ -367,7 +382,7 @@ std::string check_batch_plan(uint32_t m, const std::vector<int32_t>& level, cons
         const uint32_t lo = pl.chunk[i], hi = pl.chunk[i + 1];
         if (hi <= lo || hi - lo > 8 || pl.item_level[hi - 1] != pl.item_level[lo]) return "bad chunk";
     }
-    return {};
+    return check_levels(pl);
 }
 
 std::string prepare_factor(uint32_t n, const uint32_t* colptr, const uint32_t* rowidx, const float* vals,
@@ -635,6 +650,9 @@ std::string prepare_factor(uint32_t n, const uint32_t* colptr, const uint32_t* r
     });
     for (int dir = 0; dir < 2; ++dir)
         if (!bad[dir].empty()) return "internal sweep plan error: " + bad[dir];
+    for (size_t l = 0; l + 1 < out.level_bound.size(); ++l)
+        for (uint32_t c = out.level_bound[l]; c < out.level_bound[l + 1]; ++c)
+            if (fl[c] != static_cast<int32_t>(l)) return "internal level bound error";
     out.fwd_level = std::move(fl);
     out.bck_level = std::move(bl);
 
