@@ -1607,9 +1607,12 @@ int occ32() {
     return b0 < b1 ? b0 : b1;
 }
 
-// One cluster per column slice (kc columns).
+// One cluster per column slice (kc columns), of the tail's CTAs or of the largest
+// power of two below that keeps all clusters within the sweep's grid (one CTA a
+// slice at least). A row's sum does not depend on the cluster's size.
 template <class F, class A>
-void tail_launch(F* kernel, const tail_args<A>& a, int kc, int cluster, int flag, cudaStream_t s) {
+void tail_launch(F* kernel, const tail_args<A>& a, int kc, int cluster, int grid, int flag, cudaStream_t s) {
+    while (cluster > 1 && cluster * (a.k / kc) > grid) cluster /= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(a.k / kc) * static_cast<unsigned>(cluster));
     cfg.blockDim = dim3(kTailThreads);
@@ -1626,9 +1629,9 @@ void tail_launch(F* kernel, const tail_args<A>& a, int kc, int cluster, int flag
 }
 
 template <int KC>
-void tail32_kc(int dir, const tail_args<float>& a, bool fp16, int cluster, cudaStream_t s) {
-    if (fp16) tail_launch(k_tail32<KC, true>, a, KC, cluster, dir, s);
-    else tail_launch(k_tail32<KC, false>, a, KC, cluster, dir, s);
+void tail32_kc(int dir, const tail_args<float>& a, bool fp16, int cluster, int grid, cudaStream_t s) {
+    if (fp16) tail_launch(k_tail32<KC, true>, a, KC, cluster, grid, dir, s);
+    else tail_launch(k_tail32<KC, false>, a, KC, cluster, grid, dir, s);
 }
 
 // The tail launch's arguments of a sweep (w.tail set).
@@ -1643,14 +1646,14 @@ tail_args<T> tail_args_of(const sweep_args<T>& w) {
     return a;
 }
 
-void tail64(int dir, const sweep_args<double>& w, cudaStream_t s) {
+void tail64(int dir, const sweep_args<double>& w, int grid, cudaStream_t s) {
     tail_args<double> a = tail_args_of(w);
     a.k = 1;
-    tail_launch(k_tail64, a, 1, w.tail->cluster, dir == 0 ? kFwdSweep : kBckSweep, s);
+    tail_launch(k_tail64, a, 1, w.tail->cluster, grid, dir == 0 ? kFwdSweep : kBckSweep, s);
 }
 
 // wide: the plan is a batch plan.
-void tail32(int dir, const sweep_args<float>& w, const double* in64, bool wide, cudaStream_t s) {
+void tail32(int dir, const sweep_args<float>& w, const double* in64, bool wide, int grid, cudaStream_t s) {
     tail_args<float> a = tail_args_of(w);
     a.k = w.k; a.in64 = in64;
     a.wide = wide;
@@ -1658,9 +1661,9 @@ void tail32(int dir, const sweep_args<float>& w, const double* in64, bool wide, 
     // Up to four clusters: a row's sums and its store are on the chain of levels, so fewer columns a
     // cluster are faster (batch of k = 4, 6-regular n = 100003, forward / backward: 394 / 414 us with
     // one cluster of 4 columns, 294 / 299 with four).
-    if (w.k >= 16) tail32_kc<4>(dir, a, fp16, w.tail->cluster, s);
-    else if (w.k == 8) tail32_kc<2>(dir, a, fp16, w.tail->cluster, s);
-    else tail32_kc<1>(dir, a, fp16, w.tail->cluster, s);
+    if (w.k >= 16) tail32_kc<4>(dir, a, fp16, w.tail->cluster, grid, s);
+    else if (w.k == 8) tail32_kc<2>(dir, a, fp16, w.tail->cluster, grid, s);
+    else tail32_kc<1>(dir, a, fp16, w.tail->cluster, grid, s);
 }
 
 // The claim units a dataflow launch works off: all, or the part outside the tail.
@@ -1707,7 +1710,7 @@ int clusters_of(F* kernel, int size) {
 template <int K>
 void sweep32_dir(int dir, const sweep_args<float>& w, const double* in64, int grid, cudaStream_t s) {
     const sweep_args<float> a = outside_tail(dir, w);
-    if (dir == 1 && w.tail) tail32(dir, w, in64, false, s);
+    if (dir == 1 && w.tail) tail32(dir, w, in64, false, grid, s);
     if (a.n_items && a.n_chunks) {
         if (a.val16) {
             if (dir == 0) k_df32<0, K, true><<<grid, kSweepThreads, 0, s>>>(a, in64);
@@ -1717,7 +1720,7 @@ void sweep32_dir(int dir, const sweep_args<float>& w, const double* in64, int gr
             else          k_df32<1, K, false><<<grid, kSweepThreads, 0, s>>>(a, in64);
         }
     }
-    if (dir == 0 && w.tail) tail32(dir, w, in64, false, s);
+    if (dir == 0 && w.tail) tail32(dir, w, in64, false, grid, s);
 }
 
 }  // namespace
@@ -1734,12 +1737,12 @@ int tail_cluster_size() {
 
 void launch_sweep64(int dir, const sweep_args<double>& w, int grid, cudaStream_t s) {
     const sweep_args<double> a = outside_tail(dir, w);
-    if (dir == 1 && w.tail) tail64(dir, w, s);
+    if (dir == 1 && w.tail) tail64(dir, w, grid, s);
     if (a.n_items && a.n_chunks) {
         if (dir == 0) k_df64<0><<<grid, kSweepThreads, 0, s>>>(a);
         else          k_df64<1><<<grid, kSweepThreads, 0, s>>>(a);
     }
-    if (dir == 0 && w.tail) tail64(dir, w, s);
+    if (dir == 0 && w.tail) tail64(dir, w, grid, s);
 }
 
 void launch_sweep32(int dir, const sweep_args<float>& a, int grid, cudaStream_t s) {
@@ -1767,7 +1770,7 @@ int sweep_grid64(int num_sms) {
 template <int K>
 void sweep32_batch_dir(int dir, const sweep_args<float>& w, int grid, cudaStream_t s) {
     const sweep_args<float> a = outside_tail(dir, w);
-    if (dir == 1 && w.tail) tail32(dir, w, nullptr, true, s);
+    if (dir == 1 && w.tail) tail32(dir, w, nullptr, true, grid, s);
     if (a.n_items && a.n_chunks) {
         if (a.val16) {
             if (dir == 0) k_dw32<0, K, true><<<grid, kSweepThreads, 0, s>>>(a);
@@ -1777,7 +1780,7 @@ void sweep32_batch_dir(int dir, const sweep_args<float>& w, int grid, cudaStream
             else          k_dw32<1, K, false><<<grid, kSweepThreads, 0, s>>>(a);
         }
     }
-    if (dir == 0 && w.tail) tail32(dir, w, nullptr, true, s);
+    if (dir == 0 && w.tail) tail32(dir, w, nullptr, true, grid, s);
 }
 
 void launch_sweep32_batch(int dir, const sweep_args<float>& a, int grid, cudaStream_t s) {

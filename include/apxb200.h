@@ -103,9 +103,10 @@ void* apxb_engine_stream(apxb_engine* e);
  * sees none of its operands arrive for that long ends in APXB_ERR_TIMEOUT, up
  * to one more budget later (cluster tails look every few hundred microseconds). */
 int apxb_engine_set_spin_budget(apxb_engine* e, uint64_t ns);
-/* Blocks of the persistent sweep launches (0 = the resident grid). Any value
- * gives the same bytes; tests use it to show the result is schedule-free.
- * Batches read it when they are created. */
+/* Blocks of the persistent sweep launches (0 = the resident grid). Their
+ * cluster tails keep within it too, down to one block per column slice (at most
+ * 4). Any value gives the same bytes; tests use it to show the result is
+ * schedule-free. Batches read it when they are created. */
 int apxb_engine_set_sweep_grid(apxb_engine* e, int blocks);
 /* Device-memory budget for factors and operators created on this engine (0 = unlimited). */
 int apxb_engine_set_memory_budget(apxb_engine* e, uint64_t bytes);

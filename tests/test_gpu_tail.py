@@ -94,6 +94,39 @@ def test_sweeps_through_the_tail(eng, shape, limit, monkeypatch):
         assert np.array_equal(dZ.cpu().numpy()[:, k - 1], one), k
 
 
+@pytest.mark.parametrize("shape", ["levels_at_the_limit", "wide_then_narrow", "rows_over_a_batch"])
+def test_the_sweep_grid_sizes_the_clusters_and_not_the_bits(eng, shape):
+    """From one block a column slice (1, 2 and 4 of them at k = 1, 2 and 4) to clusters of 16."""
+    import torch
+    _, F = layered(*SHAPES[shape], seed=7)
+    D = native.DeviceFactor(eng, F)
+    D32 = native.DeviceFactor(eng, F, precision=native.PREC_FP32)
+    x = {k: torch.from_numpy(np.random.default_rng(k).standard_normal((F.m, k))).cuda() for k in (1, 2, 4, 16)}
+
+    def pairs():
+        out = []
+        for k in x:
+            z = torch.empty_like(x[k])
+            torch.cuda.synchronize()
+            D32.sweep_pair_multi(k, x[k], z)
+            eng.sync()
+            out.append(z)
+        z = torch.empty_like(x[1])
+        torch.cuda.synchronize()
+        D.sweep_pair(x[1], z)
+        eng.sync()
+        return out + [z]
+
+    want = pairs()
+    try:
+        for grid in (1, 3, 7, 8, 31, 64):
+            eng.set_sweep_grid(grid)
+            for got, ref in zip(pairs(), want):
+                assert torch.equal(got, ref), (grid, got.shape)
+    finally:
+        eng.set_sweep_grid(0)
+
+
 @pytest.mark.parametrize("k", [1, 2, 8, 16, 32])
 def test_batches_of_instances_with_and_without_tails(eng, k):
     """Instances with a tail, without one and wholly inside theirs share a batch: each gives the bytes it gives alone.
