@@ -122,21 +122,24 @@ def test_apply_sddm_is_bit_exact_and_laplacian_close(eng):
 
 
 @pytest.mark.parametrize("name", ["grid3d_48", "grid2d_256"])
-def test_serial_segment_path_is_bit_exact(eng, name, monkeypatch):
-    """The optional serial-segment launch (tiny trailing levels solved by one
-    block through shared memory) gives the same bytes as the dataflow path."""
+def test_tail_level_limits_are_bit_exact(eng, name, monkeypatch):
+    """The narrow last levels in a cluster tail, at the default limit of rows a
+    level, at a small one and without a tail: the same bytes in fp64."""
     A, F = problem(name)
     O = oracle.Oracle(A, F)
-    monkeypatch.setenv("APXB_SEG_LEVEL_ROWS", "64")
-    D = native.DeviceFactor(eng, F)
-    D32 = native.DeviceFactor(eng, F, precision=native.PREC_FP32)
-    monkeypatch.delenv("APXB_SEG_LEVEL_ROWS")
-    D64_plain = native.DeviceFactor(eng, F, precision=native.PREC_FP32)
     x = np.random.default_rng(6).standard_normal(F.m)
-    assert np.array_equal(_pair_dev(eng, D, x), O.pair(x))
-    z32 = _pair_dev(eng, D32, x)
     want = O.pair(x)
-    assert np.linalg.norm(z32 - want) / np.linalg.norm(want) < FP32_SWEEP_RTOL
+    for limit in (None, "64", "0"):
+        if limit is not None:
+            monkeypatch.setenv("APXB_SEG_LEVEL_ROWS", limit)
+        D = native.DeviceFactor(eng, F)
+        D32 = native.DeviceFactor(eng, F, precision=native.PREC_FP32)
+        for grid in (1, 7, 0):
+            eng.set_sweep_grid(grid)
+            assert np.array_equal(_pair_dev(eng, D, x), want), (limit, grid)
+            z32 = _pair_dev(eng, D32, x)
+            assert np.linalg.norm(z32 - want) / np.linalg.norm(want) < FP32_SWEEP_RTOL, (limit, grid)
+        eng.set_sweep_grid(0)
 
 
 RZ_RTOL = 1e-12   # r.z: the same products, summed in another (fixed) association than the reference's
