@@ -62,7 +62,7 @@ struct sweep_args {
     const double* rhs_sub;            // nullable: device scalar(s) subtracted from every rhs
     T* out;                           // tracked solution [row][k]
     T* reset;                         // nullable: re-armed at every solved row
-    T* copy_out;                      // nullable: untracked copy of the solution
+    T* copy_out;                      // nullable: untracked copy of the solution (fp64 sweeps)
     sweep_ctl* ctl;
     dev_error* err;
     const int* skip;                  // nullable: the launch is a no-op when *skip != 0

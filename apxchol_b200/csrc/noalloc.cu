@@ -68,6 +68,8 @@ int scratch_on(int device, double** out) {
     return APXB_OK;
 }
 
+// No cluster tail: this pair keeps every level in the dataflow launches, as it
+// was made (same bytes either way; a tail would need no memory).
 apxb::sweep_args<double> noalloc_args(const apxb_factor* f, int dir, apxb::sweep_ctl* ctl) {
     apxb::sweep_args<double> a{};
     plan_args(f, dir, a);

@@ -200,12 +200,13 @@ struct stage_desc {
     uint32_t info, row, q, e;
 };
 
-template <class T>
-__device__ __forceinline__ void load_desc(const sweep_args<T>& a, unsigned c, stage_desc& d) {
+// Descriptor of item c (nothing for c >= end); args: sweep_args or tail_args.
+template <class A>
+__device__ __forceinline__ void load_desc(const A& a, unsigned c, unsigned end, stage_desc& d) {
     const unsigned lane = threadIdx.x & 31u;
     d.c = c;
     d.info = 0; d.row = kNoRowDev; d.q = 0; d.e = 0;
-    if (c < a.n_items) {
+    if (c < end) {
         const size_t pos = static_cast<size_t>(c) * 32 + lane;
         d.info = __ldg(a.info + c);
         d.row = __ldg(a.ord + pos);
@@ -217,7 +218,6 @@ __device__ __forceinline__ void load_desc(const sweep_args<T>& a, unsigned c, st
 // Lane view of an item after stage D: the lane's group, its row, and its range.
 struct lane_view {
     unsigned c, lg, G, u, gid;
-    unsigned rows;          // rows of the item
     bool valid, thin;
     uint32_t row, q, len;   // off-diagonals at [q, q + len); diagonal at q + len
 };
@@ -226,7 +226,6 @@ __device__ __forceinline__ lane_view view_of(const stage_desc& d) {
     const unsigned lane = threadIdx.x & 31u;
     lane_view v;
     v.c = d.c;
-    v.rows = d.info & 0xffu;
     v.lg = (d.info >> 8) & 0xffu;
     v.G = 1u << v.lg;
     v.u = lane & (v.G - 1u);
@@ -311,19 +310,6 @@ __device__ __forceinline__ void load_data64(const sweep_args<double>& a, const s
     }
 }
 
-// Where the rows' operands are read and how a warp waits for them.
-struct far_src64 {
-    const sweep_args<double>& a;
-    int where;
-    bool back;                      // the newest dependency comes first (backward plans), else last
-    idle_clock clk;
-    __device__ __forceinline__ void load(bool on, uint32_t j, double& y) const { ld_if(on, a.out + j, y); }
-    __device__ __forceinline__ bool idle(uint32_t row) { return clk.idle(a.err, a.budget_ns, where, row); }
-    template <class Moved>
-    __device__ __forceinline__ bool idle(uint32_t row, Moved&& moved) { return clk.idle(a.err, a.budget_ns, where, row, moved); }
-    __device__ __forceinline__ void progress() { clk.spins = 0; }
-};
-
 // A lane waits on its newest pending operand alone, kLight polls at a time
 // between passes over all of them: what it waits for last arrives last, and
 // every poll of every waiting warp is a load that the working warps' loads
@@ -346,7 +332,7 @@ __device__ __forceinline__ V pick(const V (&v)[B], int k) {
 // product of an operand that has arrived into shared memory (prod: 32 doubles a
 // step, the warp's own), and every group consumes its leading entries.
 template <unsigned LG>
-__device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, double* prod, double& total) {
+__device__ __forceinline__ bool run_group64(const sweep_args<double>& a, int where, bool back, stage_data64& s, double* prod, double& total) {
     constexpr unsigned G = 1u << LG;
     const lane_view& v = s.v;
     const unsigned lane = threadIdx.x & 31u;
@@ -355,12 +341,13 @@ __device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, dou
     const uint32_t gend = v.thin ? (v.len & ~3u) : v.len;   // entries the chains take
     double sum = 0.0;
     uint32_t at = 0;
+    idle_clock clk;
     for (uint32_t jb = 0; jb < Jmax; jb += kBatch) {
         if (jb > 0) {
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
                 const uint32_t t = ((jb + k) << LG) + v.u;
-                if (t < v.len) { s.jj[k] = __ldg(src.a.idx + v.q + t); s.ww[k] = __ldg(src.a.val + v.q + t); }
+                if (t < v.len) { s.jj[k] = __ldg(a.idx + v.q + t); s.ww[k] = __ldg(a.val + v.q + t); }
             }
             __syncwarp();   // the last batch's products have been read
         }
@@ -370,7 +357,7 @@ __device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, dou
         for (int k = 0; k < kBatch; ++k) {
             const bool on = ((jb + k) << LG) + v.u < v.len;
             y[k] = sent_of(0.0);
-            src.load(on, s.jj[k], y[k]);
+            ld_if(on, a.out + s.jj[k], y[k]);
             pend |= on ? 1u << k : 0u;
         }
         for (;;) {
@@ -398,12 +385,12 @@ __device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, dou
                     chain_to<LG, 1>(pr, jb, 0, upto, at, sum);
                 }
                 if (!open) break;
-                if (__any_sync(kFull, at != from)) src.progress();
-                else if (src.idle(v.row)) return false;
+                if (__any_sync(kFull, at != from)) clk.spins = 0;
+                else if (clk.idle(a.err, a.budget_ns, where, v.row)) return false;
                 if (light == kLight) break;
-                const int kn = newest_of(pend, src.back);
+                const int kn = newest_of(pend, back);
                 double w = sent_of(0.0);
-                src.load(pend != 0, pick(s.jj, kn), w);
+                ld_if(pend != 0, a.out + pick(s.jj, kn), w);
                 if (pend && !is_sent(w)) {
                     prod[32 * kn + lane] = __dmul_rn(static_cast<double>(pick(s.ww, kn)), w);
                     pend &= ~(1u << kn);
@@ -411,7 +398,7 @@ __device__ __forceinline__ bool run_group64(far_src64& src, stage_data64& s, dou
             }
             if (!open) break;
 #pragma unroll
-            for (int k = 0; k < kBatch; ++k) src.load((pend >> k) & 1u, s.jj[k], y[k]);
+            for (int k = 0; k < kBatch; ++k) ld_if((pend >> k) & 1u, a.out + s.jj[k], y[k]);
         }
     }
     const double s1 = __shfl_sync(kFull, sum, 1, static_cast<int>(G));
@@ -454,14 +441,15 @@ __device__ __forceinline__ double lane_sum64(const double (&p)[kBatch], uint32_t
 
 // One lane per row (<= kBatch off-diagonals): all operands, then the sum in
 // straight line.
-__device__ __forceinline__ bool run_lane64(far_src64& src, stage_data64& s, double& total) {
+__device__ __forceinline__ bool run_lane64(const sweep_args<double>& a, int where, stage_data64& s, double& total) {
     const lane_view& v = s.v;
     const uint32_t n = v.len;   // <= kBatch for these rows
     double y[kBatch];
+    idle_clock clk;
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
         y[k] = sent_of(0.0);
-        src.load(static_cast<uint32_t>(k) < n, s.jj[k], y[k]);
+        ld_if(static_cast<uint32_t>(k) < n, a.out + s.jj[k], y[k]);
     }
     for (;;) {
         bool open = false;
@@ -474,9 +462,9 @@ __device__ __forceinline__ bool run_lane64(far_src64& src, stage_data64& s, doub
             for (int k = 0; k < kBatch; ++k) p |= static_cast<uint32_t>(k) < n && is_sent(y[k]) ? 1u << k : 0u;
             return pending_changed(row, 0, p);
         };
-        if (src.idle(v.row, moved)) return false;
+        if (clk.idle(a.err, a.budget_ns, where, v.row, moved)) return false;
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) src.load(static_cast<uint32_t>(k) < n && is_sent(y[k]), s.jj[k], y[k]);
+        for (int k = 0; k < kBatch; ++k) ld_if(static_cast<uint32_t>(k) < n && is_sent(y[k]), a.out + s.jj[k], y[k]);
     }
     double p[kBatch];
 #pragma unroll
@@ -487,13 +475,13 @@ __device__ __forceinline__ bool run_lane64(far_src64& src, stage_data64& s, doub
 
 // The off-diagonal sums of one item's rows in the reference's order. Returns
 // false when the warp must drain.
-__device__ __forceinline__ bool run_rows64(far_src64& src, stage_data64& s, double* prod, double& total) {
+__device__ __forceinline__ bool run_rows64(const sweep_args<double>& a, int where, bool back, stage_data64& s, double* prod, double& total) {
     switch (s.v.lg) {
-        case 0: return run_lane64(src, s, total);
-        case 2: return run_group64<2>(src, s, prod, total);
-        case 3: return run_group64<3>(src, s, prod, total);
-        case 4: return run_group64<4>(src, s, prod, total);
-        default: return run_group64<5>(src, s, prod, total);
+        case 0: return run_lane64(a, where, s, total);
+        case 2: return run_group64<2>(a, where, back, s, prod, total);
+        case 3: return run_group64<3>(a, where, back, s, prod, total);
+        case 4: return run_group64<4>(a, where, back, s, prod, total);
+        default: return run_group64<5>(a, where, back, s, prod, total);
     }
 }
 
@@ -504,8 +492,7 @@ __device__ __forceinline__ bool run64(const sweep_args<double>& a, stage_data64&
     const lane_view& v = s.v;
     double total = 0.0;
     const recip64 inv = recip_of(s.d);
-    far_src64 src{a, DIR == 0 ? kFwdSweep : kBckSweep, DIR == 1, {}};
-    if (!run_rows64(src, s, prod, total)) return false;
+    if (!run_rows64(a, DIR == 0 ? kFwdSweep : kBckSweep, DIR == 1, s, prod, total)) return false;
     if (v.valid && v.u == 0) {
         double rhs = s.rhs;
         if (a.rhs_sub) rhs = __dsub_rn(rhs, *a.rhs_sub);
@@ -530,16 +517,16 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_df64(const sweep_args<doub
     chunk_claim cc;
     cc.start(a);
     stage_desc dD;
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     stage_data64 sL;
     load_data64(a, dD, sL);
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     int bad = 0;   // the error word, read one item late so the load is never waited on
     while (sL.v.c < a.n_items) {
         // rotate: run L, data for D, descriptor of the next claimed item
         stage_data64 sR = sL;
         load_data64(a, dD, sL);
-        load_desc(a, cc.next(a), dD);
+        load_desc(a, cc.next(a), a.n_items, dD);
         if (__shfl_sync(kFull, bad, 0)) break;
         if (lane == 0) bad = ld_relaxed_int(&a.err->code);
         if (!run64<DIR>(a, sR, prod)) break;
@@ -808,15 +795,15 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_df32(const sweep_args<floa
     chunk_claim cc;
     cc.start(a);
     stage_desc dD;
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     stage_data32<K> sL;
     load_data32<DIR, K, H>(a, in64, dD, sL);
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     int bad = 0;   // the error word, read one item late
     while (sL.v.c < a.n_items) {
         stage_data32<K> sR = sL;
         load_data32<DIR, K, H>(a, in64, dD, sL);
-        load_desc(a, cc.next(a), dD);
+        load_desc(a, cc.next(a), a.n_items, dD);
         if (__shfl_sync(kFull, bad, 0)) break;
         if (lane == 0) bad = ld_relaxed_int(&a.err->code);
         if (!run32<DIR, K, H>(a, sR)) break;
@@ -981,15 +968,15 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_dw32(const sweep_args<floa
     chunk_claim cc;
     cc.start(a);
     stage_desc dD;
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     stage_wide<K> sL;
     load_wide<K, H>(a, dD, sL);
-    load_desc(a, cc.next(a), dD);
+    load_desc(a, cc.next(a), a.n_items, dD);
     int bad = 0;   // the error word, read one item late so the load is never waited on
     while (sL.v.c < a.n_items) {
         stage_wide<K> sR = sL;
         load_wide<K, H>(a, dD, sL);
-        load_desc(a, cc.next(a), dD);
+        load_desc(a, cc.next(a), a.n_items, dD);
         if (__shfl_sync(kFull, bad, 0)) break;
         if (lane == 0) bad = ld_relaxed_int(&a.err->code);
         if (!run_wide<DIR, K, H>(a, sR, sL)) break;
@@ -1008,8 +995,10 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_dw32(const sweep_args<floa
 // costs a store, an L2 round trip and the polls of every warp that waits
 // further down (0.7 us alone, 1.1 us and more with the whole grid polling);
 // here a hop is a DSM store and a shared-memory poll, and no other SM sees it.
-// What is left of a hop (0.45 us in fp32) is the instructions between the
-// operand's arrival and the store, so those paths are short: a row's lanes all
+// What is left of a hop (chains of one-row levels: 0.45 us in fp32, 0.61 in fp64,
+// against 0.68 and 0.83 in the dataflow kernels; levels of some hundred rows,
+// 6-regular n = 100003: 0.56 in fp32) is the instructions between the operand's
+// arrival and the store, so those paths are short: a row's lanes all
 // hold its sum, right-hand side and divisor, the batches of a row are compiled
 // for 1, 2, 4 and 8 steps, the divisor's reciprocal, the store addresses and
 // everything else that does not depend on the operands are ready before.
@@ -1117,21 +1106,6 @@ __device__ __forceinline__ tail_seat take_seat(int kc, unsigned base) {
     t.warps = cs * (kTailThreads / 32);
     t.base = base;
     return t;
-}
-
-// Descriptor of item c of the tail (nothing for c >= item1).
-template <class T>
-__device__ __forceinline__ void tail_desc(const tail_args<T>& p, uint32_t c, stage_desc& d) {
-    const unsigned lane = threadIdx.x & 31u;
-    d.c = c;
-    d.info = 0; d.row = kNoRowDev; d.q = 0; d.e = 0;
-    if (c < p.item1) {
-        const size_t pos = static_cast<size_t>(c) * 32 + lane;
-        d.info = __ldg(p.info + c);
-        d.row = __ldg(p.ord + pos);
-        d.q = __ldg(p.ptr + pos);
-        d.e = __ldg(p.ptr + pos + 1);
-    }
 }
 
 // Lane view of a tail item: a factor plan's rows take all 32 lanes (its lane
@@ -1330,11 +1304,11 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail64(const tail_args<doub
     stage_desc ds;
     near_row64 s0, s1;
     double y0[kBatch], y1[kBatch];
-    tail_desc(a, c, ds);
+    load_desc(a, c, a.item1, ds);
     near_data64(a, ds, s0);
-    tail_desc(a, c + t.warps, ds);
+    load_desc(a, c + t.warps, a.item1, ds);
     near_data64(a, ds, s1);
-    tail_desc(a, c + 2 * t.warps, ds);
+    load_desc(a, c + 2 * t.warps, a.item1, ds);
     near_outside64(a, s0, y0);
     while (s0.v.c < a.item1) {
         near_outside64(a, s1, y1);   // the next item's indices came in with the last one
@@ -1356,7 +1330,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail64(const tail_args<doub
         for (int k = 0; k < kBatch; ++k) y0[k] = y1[k];
         near_data64(a, ds, s1);
         c += t.warps;
-        tail_desc(a, c + 2 * t.warps, ds);
+        load_desc(a, c + 2 * t.warps, a.item1, ds);
     }
     cluster_barrier();   // no CTA leaves while another may still store into its copy
 }
@@ -1545,11 +1519,11 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail32(const tail_args<floa
     stage_desc ds;
     near_row32<KC> s0, s1;
     float y0[kBatch][KC], y1[kBatch][KC];
-    tail_desc(a, c, ds);
+    load_desc(a, c, a.item1, ds);
     near_data32<KC, H>(a, t, ds, back, s0);
-    tail_desc(a, c + t.warps, ds);
+    load_desc(a, c + t.warps, a.item1, ds);
     near_data32<KC, H>(a, t, ds, back, s1);
-    tail_desc(a, c + 2 * t.warps, ds);
+    load_desc(a, c + 2 * t.warps, a.item1, ds);
     near_outside32<KC>(a, t, s0, y0);
     while (s0.v.c < a.item1) {
         near_outside32<KC>(a, t, s1, y1);   // the next item's indices came in with the last one
@@ -1578,7 +1552,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail32(const tail_args<floa
             for (int r = 0; r < KC; ++r) y0[k][r] = y1[k][r];
         near_data32<KC, H>(a, t, ds, back, s1);
         c += t.warps;
-        tail_desc(a, c + 2 * t.warps, ds);
+        load_desc(a, c + 2 * t.warps, a.item1, ds);
     }
     cluster_barrier();   // no CTA leaves while another may still store into its copy
 }
