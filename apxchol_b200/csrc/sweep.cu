@@ -696,11 +696,12 @@ __device__ __forceinline__ void load_data32(const sweep_args<float>& a, const do
 //  * from 2 columns on a lane consumes its rows as they arrive and polls only
 //    those from the first missing one on (the wider polls cost what the vote
 //    saves), by predicate up to 4 columns and by branch from 8 on.
-// One pair of sweeps, all levels in the dataflow launches, us, straight line ->
-// this rule, mean of seven placements of the factor: R-MAT-14 k = 4 777 -> 734,
-// k = 8 1101 -> 887, k = 16 1807 -> 1532; 6-regular n = 100003 1641 -> 1563,
-// 2288 -> 1880, 3793 -> 3307; 96^3 grid 671 -> 630, 934 -> 803, 1401 -> 1314.
-// At one column in order against straight line: 758 : 724, 2204 : 2125, 754 : 732.
+// One pair of sweeps, all levels in the dataflow launches, us, straight line for
+// all -> this rule, mean of seven placements of the factor: R-MAT-14 k = 4
+// 773 -> 743, k = 8 1074 -> 894, k = 16 1740 -> 1486; 6-regular n = 100003
+// 1635 -> 1549, 2283 -> 1889, 3747 -> 3089; 96^3 grid 670 -> 621, 924 -> 797,
+// 1396 -> 1258; k = 2 the same within 1.5 % (96^3 grid 653 -> 629). At one column
+// in order against straight line: 758 : 724, 2204 : 2125, 754 : 732.
 template <int B, int K>
 __device__ __forceinline__ bool gather32(const sweep_args<float>& a, int where, uint32_t row, uint32_t batch, idle_clock& clk, uint32_t nk,
                                          const uint32_t (&jj)[B], const float (&ww)[B], float (&yv)[B][K], float (&acc)[K]) {
