@@ -335,9 +335,9 @@ int apxb_test_stalled_launch(apxb_engine* e, apxb_factor* f, int dir, int k, int
  * storage on the device (the reference does this work on the host:
  * cuda.h:280-420, cuda_host.h:66-558). This hook prepares the given factor
  * both ways and compares every array: CSC(L11) and CSR(L11) after the drop,
- * levels, row sum modes, both directions' sweep plans, the batch plans for
- * k right-hand sides (k > 0) and, when the operator is given (full symmetric
- * CSC, int32), its permutation P A P^T (pcg_cuda.h:304-404). APXB_OK when
+ * levels, row sum modes, both directions' sweep plans with their level tables,
+ * the batch plans for k right-hand sides (k > 0) and, when the operator is given
+ * (full symmetric CSC, int32), its permutation P A P^T (pcg_cuda.h:304-404). APXB_OK when
  * all are identical (or both preparations reject the input with the same
  * message); else APXB_ERR_INVALID naming the first array that differs. */
 int apxb_test_prep_compare(apxb_engine* e, uint32_t n, const uint32_t* colptr, const uint32_t* rowidx,
